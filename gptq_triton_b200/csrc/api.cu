@@ -23,6 +23,8 @@ static int g_soft_max_splits = 8;  // the planner avoids more splits than this (
 static int g_qa_stages = 2;       // ring depth of the attention-block kernel (gptq_debug_qa_stages); 7B step, gate/up at 3 stages: 4 / 3 / 2 stages 589 / 596 / 600 tokens/s at 2.1 k context, 453 / 457 / 457 at 8 k, 660 / 676 / 681 at 300
 static int g_pdl = 1;             // programmatic dependent launch for the decode-step kernels (+3 % on the decode step)
 
+bool pdl_enabled() { return g_pdl != 0; }      // for the launchers in the other files
+
 static int sm_count() {
 	static int cached[64] = {0};
 	int dev = 0;

@@ -1,25 +1,36 @@
 // Prefill-regime (M > 16) quantised matmul on the 5th-generation tensor cores of sm_100a.
 //
-// Y[M,N] = X[M,K] · deq(W)[K,N] with fp16 operands and fp32 accumulation in tensor memory.
-// One CTA computes a 128 or 256 (rows of X) x 128 or 256 (columns of W) tile; K advances in blocks
-// of 64.  256-row tiles issue two M = 128 MMAs per K step against the same dequantised B stage.
+// The product is computed transposed, Y^T = deq(W)^T X^T: a weight column is a lane of tensor memory and the rows of X are the N
+// of the MMA.  The dequantised weights are the A operand in TENSOR MEMORY, X is the B operand in shared memory.
+//   - A thread that owns a column writes the 64 weights of a K-block with one tcgen05.st: no shared-memory stores, no proxy fence.
+//     With both operands in shared memory the operand traffic was the bound of long prompts (176 KB per 256 x 256 x 64 block at
+//     128 bytes per clock).
+//   - The N of an MMA is any multiple of 16 up to 256, so a tile holds exactly the rows that there are: 40 rows cost 48, not 128.
+// A CTA computes 128 columns (64 gate + 64 up columns for the fused MLP) x nr rows; K advances in blocks of 64.
 //
-//   warp 0      TMA producer: X tile [128 x 64] fp16, K-major, 128-byte swizzle (one thread)
-//   warp 1      MMA issuer: tcgen05.mma.cta_group::1.kind::f16, M=128 N=128 K=16, four per
-//               K-block (eight with the second weight stream), tcgen05.commit frees the stage;
-//               the warp also owns the TMEM allocation
-//   warps 2-17  dequantise, four groups of four warps, group j serving K-blocks j, j+4, ...: a
-//               thread owns a weight column of the tile, reads the K-block's 8 packed words of that
-//               column from a TMA-fed ring, turns each into 8 fp16 weights
-//               (q - zero) * scale with ONE rounding — the fp16 weight of the
-//               dequantise-then-matmul path — and stores them as one 16-byte unit of the
-//               K-major, 128-byte-swizzled B tile; fence.proxy.async + mbarrier arrive.
-//               After the last K-block the same warps drain TMEM (tcgen05.ld 32x32b) and run
-//               the epilogue: bias/residual, SiLU(gate)*up, or rotary + scatter to Q/K/V.
+//   warp 0      packed weights (8 words x 128 columns per K-block), scales and zeros by TMA / bulk copies into a deep ring
+//   warp 1      X tile [nr x 64] fp16, K-major, 128-byte swizzle
+//   warp 2      MMA issuer: tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, M = 128, N = nr, K = 16; one wait and one
+//               commit per stage of one or two K-blocks
+//   warp 3      owns the tensor-memory allocation (nr columns of accumulators, 4 to 8 stages of 32 or 64 columns of weights)
+//   warps 4-19  dequantise, four groups of four warps, group j serving the stages j, j + 4, ...: 8 packed words of a column
+//               become 64 fp16 weights (q - zero) * scale with ONE rounding each, the weights of the dequantise-then-matmul path
+// Afterwards the accumulators are turned through shared memory into an fp32 tile [row][128] and all warps run the epilogue:
+// bias / residual, SiLU(gate) * up, or rotary + scatter to Q / K / V.
+// Split K: the CTAs of a cluster take consecutive ranges of K-blocks of one tile; each then finishes its share of the rows,
+// reading the partial tiles of the others from their shared memory in split order (deterministic; no pass through global memory).
 //
-// Every mbarrier wait is bounded; a wait that runs out sets a status word and the kernel
-// unwinds (TMEM is still released).
+// What bounds it: up to about 130 rows the issue slots of the dequantisation (17 instructions per 8 weights), above the MMAs and, from
+// about 1000 rows, the power limit (1250 - 1430 TFLOP/s; cuBLAS bf16: 1670 in a burst, 1410 sustained).  Measured, in brackets the
+// kernel with both operands in shared memory that this one replaced (us; 128-row tiles, split K through global memory):
+//   M = 17    4096 -> 12288  12.3 (26.3)   22016 -> 8192  30.4 (56.2)   gate/up 8192 -> 2 x 22016   69 (190)
+//   M = 203   4096 -> 12288  22.1 (46.8)   22016 -> 8192  58.5 (84.2)   gate/up 8192 -> 2 x 22016  126 (247)
+//   M = 512   4096 -> 4096   17.0 (36.0)   11008 -> 4096  36.3 (55.8)   gate/up 4096 -> 2 x 11008   86 (132)
+//   M = 2048  4096 -> 4096   53.2 (58.0)   11008 -> 4096   134 (145)    gate/up 4096 -> 2 x 11008  296 (332)
+//
+// Every mbarrier wait is bounded; a wait that runs out sets a status word and the kernel unwinds (tensor memory is still released).
 #include <algorithm>
+#include <atomic>
 
 #include <cuda.h>
 
@@ -30,29 +41,87 @@ namespace gptq {
 
 namespace {
 
-constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64, TC_STAGES = 4;
-constexpr int TC_WORKERS = 512;                             // dequantise / epilogue threads: 4 groups x 4 warps
-constexpr int TC_THREADS = 64 + TC_WORKERS;
-constexpr int TC_TILE_BYTES = TC_BM * TC_BK * 2;            // 16 KB: one A or B stage
+constexpr int TC_BK = 64;
+constexpr int TC_THREADS = 128 + 512;                       // producers, issuer, tensor-memory owner; 16 dequantise warps
+constexpr int TC_MAX_NR = 256;                              // rows per tile (N of the MMA)
+constexpr int TC_PAIR_NR = 144;                             // two K-blocks per stage up to this many rows (four stages fit)
+constexpr int TC_TMEM_COLS = 512;
+constexpr int TC_GROUPS = 4;                                // dequantise groups
+// a packed stage of kp K-blocks: 8 kp words of 128 columns, scales and zeros of every K-block
+__host__ __device__ constexpr int TC_W_SC(int kp) { return 4096 * kp; }
+__host__ __device__ constexpr int TC_W_QZ(int kp) { return TC_W_SC(kp) + 256 * kp; }
+__host__ __device__ constexpr int TC_W_STAGE(int kp) { return (TC_W_QZ(kp) + 64 * kp + 127) / 128 * 128; }
+constexpr int TC_MAX_STAGES = 8, TC_MAX_WSTAGES = 20;
+constexpr int TC_BARS = 2 * TC_MAX_STAGES + 2 * TC_MAX_WSTAGES + 1;
+constexpr int TC_BAR_BYTES = (TC_BARS + 1) * 8;
+constexpr int TC_SMEM = 227 * 1024;
 constexpr uint32_t TC_SPIN = 1u << 24;
-// pipeline depth by tile configuration (shared memory: S * (MH * 16 KB + NSTREAM * BN * 128 B) + packed ring)
-__host__ __device__ constexpr int tc_stages(int nstream, int bn, int mh) { return (mh == 2 && nstream * bn == 256) ? 3 : TC_STAGES; }
-__host__ __device__ constexpr int tc_pstages(int nstream, int bn, int mh) { return (mh == 2) ? (nstream * bn == 256 ? 3 : 6) : (nstream * bn == 256 ? 4 : 8); }
+static_assert(4 * TC_MAX_NR * TC_BK * 2 + 16 * TC_W_STAGE(1) + TC_BAR_BYTES <= TC_SMEM, "shared memory per CTA, one K-block per stage");
+static_assert(4 * TC_PAIR_NR * TC_BK * 2 * 2 + 8 * TC_W_STAGE(2) + TC_BAR_BYTES <= TC_SMEM, "shared memory per CTA, two");
+static_assert(TC_MAX_NR + 4 * (TC_BK / 2) <= TC_TMEM_COLS && TC_PAIR_NR + 4 * TC_BK <= TC_TMEM_COLS, "tensor memory");
 
 struct TcParams {
 	TcArgs a;
-	int epi;
 	int *status;
-	int kb_per_split;            // K-blocks of 64 per CTA along grid.z (all of them without split-K)
-	float *partial;              // split-K: [split][M][N] fp32 partial sums in the workspace, else nullptr
+	int nr;                      // rows per tile
+	int kb_per_split;            // K-blocks per CTA
+	int s_stages, w_stages;      // ring depths: X / dequantised weights (4 .. 8), packed weights (a multiple of 4)
+	int bar_off;
+	int out8;                    // rotary outputs may be stored 8 bytes at a time
 };
 
-}   // namespace
+// Wait of a whole warp: one poll inline, the bounded loop and the look at the abort flag out of line.  Every lane gets the same answer.
+__device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+	return __all_sync(0xffffffffu, !*abort_flag && mbar_wait_bounded(bar, parity, TC_SPIN));
+}
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+	return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || tc_wait_slow(bar, parity, abort_flag);
+}
+// the same without a call, for code with many live registers
+__device__ __forceinline__ bool tc_wait_inline(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+	if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+	return __all_sync(0xffffffffu, !*abort_flag && mbar_wait_bounded(bar, parity, TC_SPIN));
+}
+__device__ __forceinline__ bool tc_elect() {
+	uint32_t r;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+	return r != 0;
+}
+__device__ __forceinline__ void tc_bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint32_t tc_lds32(uint32_t addr) {
+	uint32_t r;
+	asm volatile("ld.shared.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
+	return r;
+}
+__device__ __forceinline__ uint32_t tc_lds16(uint32_t addr) {
+	unsigned short r;
+	asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(addr) : "memory");
+	return r;
+}
+__device__ __forceinline__ float4 tc_lds128(uint32_t addr) {
+	float4 r;
+	asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(addr) : "memory");
+	return r;
+}
+// four floats at this CTA's address `addr`, in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ float4 tc_ld_peer(uint32_t addr, uint32_t rank) {
+	float4 r;
+	asm volatile(
+		"{\n\t.reg .b32 a;\n\t"
+		"mapa.shared::cluster.u32 a, %4, %5;\n\t"
+		"ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n\t}"
+		: "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w)
+		: "r"(addr), "r"(rank)
+		: "memory");
+	return r;
+}
+__device__ __forceinline__ void tc_cluster_sync() {
+	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
-// forward declaration of the kernel body (second half of this file)
-template <int NSTREAM, int EPI, int BN, int MH>
-__global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant__ CUtensorMap tmx, const __grid_constant__ CUtensorMap tmw0,
-														   const __grid_constant__ CUtensorMap tmw1, const TcParams p);
+}   // namespace
 
 }   // namespace gptq
 
@@ -62,34 +131,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 namespace gptq {
 
 EncodeTiledFn tensor_map_encoder();      // defined in api.cu
-int g_tc_force = 0;                    // tests: 0 = choose by cost, 1 = 128 x 128, 2 = 128 x 256, 3 = 256 x 256 (256 x 128 for two streams), 4 = 256 x 128
-constexpr double TC_SPEED_256x128 = 1.6;
+bool pdl_enabled();
+int g_tc_force = 0;                    // tests: 0 = choose by cost, 1 .. 4 = at most 64, 128, 192, 256 rows per tile
 extern "C" void gptq_debug_tc_force(int cfg) { g_tc_force = cfg; }
 
 bool tc_shape_ok(int M, int K, int N, int groupsize) {
-	return M > 16 && N % TC_BN == 0 && K % TC_BK == 0 && groupsize % TC_BK == 0 && K % groupsize == 0;
+	return M > 16 && N % 128 == 0 && K % TC_BK == 0 && groupsize % TC_BK == 0 && K % groupsize == 0;
 }
 
-// Workspace: the status word at the end of the first 16 KB; behind it room for the fp32 partial sums of a split-K
-// launch (up to TC_MAX_SPLITK splits of M x N, at most TC_SPLIT_BYTES: larger problems fill the chip without it).
-constexpr int TC_MAX_SPLITK = 4;
-constexpr size_t TC_SPLIT_BYTES = (size_t)96 << 20;
-size_t tc_ws_bytes(int M, int N) {
-	const size_t part = (size_t)TC_MAX_SPLITK * (size_t)std::max(M, 0) * (size_t)std::max(N, 0) * 4;
-	return 16384 + (M > 16 && part <= TC_SPLIT_BYTES ? part : 0);
-}
-int g_tc_splitk = 0;                   // tests: 0 = choose by cost, n = force n splits where the epilogue allows
+size_t tc_ws_bytes(int, int) { return 16384; }      // the status word at the end of the first 16 KB
+int g_tc_splitk = 0;                   // tests: 0 = choose by cost, n = force n splits
 extern "C" void gptq_debug_tc_splitk(int n) { g_tc_splitk = n; }
 
-static int x_tensor_map(const __half *x, int M, int K, long long ldx, CUtensorMap *out) {
+static int tc_map(const void *base, CUtensorMapDataType type, int elem, cuuint64_t cols, cuuint64_t rows, cuuint64_t ld, cuuint32_t box_cols, cuuint32_t box_rows,
+				  CUtensorMapSwizzle swizzle, CUtensorMap *out) {
 	EncodeTiledFn enc = tensor_map_encoder();
 	if (!enc) return GPTQ_ERR_CUDA;
-	cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-	cuuint64_t strides[1] = {(cuuint64_t)ldx * 2};
-	cuuint32_t box[2] = {TC_BK, TC_BM};
-	cuuint32_t estr[2] = {1, 1};
-	CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-					 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	cuuint64_t dims[2] = {cols, rows}, strides[1] = {ld * elem};
+	cuuint32_t box[2] = {box_cols, box_rows}, estr[2] = {1, 1};
+	CUresult r = enc(out, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+					 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 	if (r != CUDA_SUCCESS) {
 		g_last_cuda_error = (int)r;
 		return GPTQ_ERR_CUDA;
@@ -97,138 +158,146 @@ static int x_tensor_map(const __half *x, int M, int K, long long ldx, CUtensorMa
 	return GPTQ_OK;
 }
 
-// Tensor map over packed weights int32 [K/8, N]: box bn columns x 8 packed rows (one K-block), no swizzle.
-static int w_tensor_map(const int32_t *qw, int K, int N, int bn, CUtensorMap *out) {
-	EncodeTiledFn enc = tensor_map_encoder();
-	if (!enc) return GPTQ_ERR_CUDA;
-	cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)(K / 8)};
-	cuuint64_t strides[1] = {(cuuint64_t)N * 4};
-	cuuint32_t box[2] = {(cuuint32_t)bn, 8};
-	cuuint32_t estr[2] = {1, 1};
-	CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<int32_t *>(qw), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-					 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-	if (r != CUDA_SUCCESS) {
-		g_last_cuda_error = (int)r;
-		return GPTQ_ERR_CUDA;
-	}
-	return GPTQ_OK;
+constexpr int TC_MAX_SPLITS = 8;       // portable cluster size
+// Estimated time of a CTA in us, fitted to measurements (M = 17 .. 2048, K = 4096 / 8192 / 11008 / 22016): a K-block costs the
+// dequantisation (0.16 us at 32 rows in stages of two, 0.22 in stages of one) or the MMAs (0.38 us at 256 rows), a tile 2.5 us to start and
+// drain; with split K the partial tiles of the cluster are summed through distributed shared memory (4.8 us at 32 rows, 7 us at 256).
+static double tc_cta_us(int nr, int splits, int kblocks) {
+	const double t_kb = nr <= TC_PAIR_NR ? 0.14 + 0.00065 * nr : std::max(0.22 + 0.0002 * nr, 0.0015 * nr);
+	return kblocks * t_kb + (splits > 1 ? 4.5 + 0.01 * nr : 2.5);
 }
 
-template <int NSTREAM, int EPI, int BN, int MH>
-static int tc_launch_inst(const CUtensorMap &tmx, const TcParams &p, cudaStream_t stream) {
-	auto k = tc_kernel<NSTREAM, EPI, BN, MH>;
-	constexpr int S = tc_stages(NSTREAM, BN, MH), PS = tc_pstages(NSTREAM, BN, MH);
-	const size_t smem = (size_t)S * (MH * TC_TILE_BYTES + NSTREAM * BN * TC_BK * 2) + (size_t)PS * NSTREAM * 8 * BN * 4 + 512;
-	static_assert((size_t)S * (MH * TC_TILE_BYTES + NSTREAM * BN * TC_BK * 2) + (size_t)PS * NSTREAM * 8 * BN * 4 + 512 <= 232448, "shared memory per CTA");
-	alignas(64) CUtensorMap tmw0, tmw1;
-	if (int rc = w_tensor_map(p.a.qw0, p.a.K, p.a.N, BN, &tmw0)) return rc;
-	if (NSTREAM == 2) {
-		if (int rc = w_tensor_map(p.a.qw1, p.a.K, p.a.N, BN, &tmw1)) return rc;
-	} else {
-		tmw1 = tmw0;
-	}
-	static bool ready[64] = {false};
-	int dev = 0;
-	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GPTQ_ERR_CUDA;
+template <int EPI, int KP>
+static int tc_ready(int dev) {
+	static std::atomic<bool> ready[64];
 	if (!ready[dev]) {
-		cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		cudaError_t e = cudaFuncSetAttribute(tc_kernel<EPI, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
 		if (e != cudaSuccess) return cuda_status(e);
 		ready[dev] = true;
 	}
-	const int nkb = p.a.K / TC_BK;
-	const int splits = (nkb + p.kb_per_split - 1) / p.kb_per_split;
-	dim3 grid(p.a.N / BN, (p.a.M + TC_BM * MH - 1) / (TC_BM * MH), splits);
-	k<<<grid, TC_THREADS, smem, stream>>>(tmx, tmw0, tmw1, p);
-	if (int rc = cuda_status(cudaGetLastError())) return rc;
-	if (p.partial) {
-		const size_t units = (size_t)p.a.M * (p.a.N / 8);
-		tc_splitk_finish<<<(unsigned)((units + 255) / 256), 256, 0, stream>>>(p.partial, splits, p.a.M, p.a.N, p.a.bias, p.a.residual, p.a.ldr, p.a.y, p.a.ldy);
-		return cuda_status(cudaGetLastError());
-	}
 	return GPTQ_OK;
+}
+
+static void tc_attrs(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int splits, bool pdl) {
+	cfg.blockDim = dim3(TC_THREADS);
+	cfg.attrs = attr;
+	cfg.numAttrs = 0;
+	if (splits > 1) {
+		cudaLaunchAttribute &c = attr[cfg.numAttrs++];
+		c.id = cudaLaunchAttributeClusterDimension;
+		c.val.clusterDim.x = 1;
+		c.val.clusterDim.y = 1;
+		c.val.clusterDim.z = splits;
+	}
+	if (pdl) {
+		cudaLaunchAttribute &c = attr[cfg.numAttrs++];
+		c.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+		c.val.programmaticStreamSerializationAllowed = 1;
+	}
+}
+
+template <int EPI, int KP>
+static int tc_go(TcParams p, int splits, int dev, cudaStream_t stream) {
+	constexpr int TN = EPI == TC_EPI_SILU ? 64 : 128;
+	const TcArgs &a = p.a;
+	if (int rc = tc_ready<EPI, KP>(dev)) return rc;
+	// rings: X and the dequantised weights share their stages, bounded by shared and by tensor memory
+	const int x_stage = p.nr * TC_BK * 2 * KP, left = TC_SMEM - TC_BAR_BYTES, w_min = KP == 2 ? 8 : 16;
+	p.s_stages = std::min({TC_MAX_STAGES, (left - w_min * TC_W_STAGE(KP)) / x_stage, (TC_TMEM_COLS - p.nr) / (KP * TC_BK / 2)});
+	p.w_stages = std::min(TC_MAX_WSTAGES, (left - p.s_stages * x_stage) / TC_W_STAGE(KP)) & ~3;
+	p.bar_off = p.s_stages * x_stage + p.w_stages * TC_W_STAGE(KP);
+	alignas(64) CUtensorMap tmx, tmw0, tmw1;
+	if (int rc = tc_map(a.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.K, a.M, a.ldx, TC_BK, p.nr, CU_TENSOR_MAP_SWIZZLE_128B, &tmx)) return rc;
+	if (int rc = tc_map(a.qw0, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.N, a.K / 8, a.N, TN, 8 * KP, CU_TENSOR_MAP_SWIZZLE_NONE, &tmw0)) return rc;
+	tmw1 = tmw0;
+	if (EPI == TC_EPI_SILU)
+		if (int rc = tc_map(a.qw1, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, a.N, a.K / 8, a.N, TN, 8 * KP, CU_TENSOR_MAP_SWIZZLE_NONE, &tmw1)) return rc;
+	cudaLaunchConfig_t cfg = {};
+	cudaLaunchAttribute attr[2];
+	tc_attrs(cfg, attr, splits, pdl_enabled());
+	cfg.stream = stream;
+	cfg.gridDim = dim3((a.M + p.nr - 1) / p.nr, a.N / TN, splits);
+	cfg.dynamicSmemBytes = p.bar_off + TC_BAR_BYTES;
+	return cuda_status(cudaLaunchKernelEx(&cfg, tc_kernel<EPI, KP>, tmx, tmw0, tmw1, p));
+}
+
+template <int EPI>
+static int tc_launch_inst(TcParams p, cudaStream_t stream) {
+	constexpr int TN = EPI == TC_EPI_SILU ? 64 : 128;
+	const TcArgs &a = p.a;
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GPTQ_ERR_CUDA;
+	if (int rc = tc_ready<EPI, 1>(dev)) return rc;
+	// CTAs that run at the same time: one per SM, in whole clusters
+	static std::atomic<int> slots[64][TC_MAX_SPLITS + 1];
+	auto slots_of = [&](int splits) -> int {
+		int n = slots[dev][splits];
+		if (n) return n;
+		if (splits == 1) {
+			if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+		} else {
+			cudaLaunchConfig_t cfg = {};
+			cudaLaunchAttribute attr[2];
+			tc_attrs(cfg, attr, splits, false);
+			cfg.gridDim = dim3(1, 1, splits);
+			cfg.dynamicSmemBytes = TC_SMEM;
+			int clusters = 0;
+			if (cudaOccupancyMaxActiveClusters(&clusters, tc_kernel<EPI, 1>, &cfg) != cudaSuccess) {
+				cudaGetLastError();
+				clusters = 0;
+			}
+			n = clusters > 0 ? clusters * splits : -1;          // -1: such clusters do not fit
+		}
+		slots[dev][splits] = n;
+		return n;
+	};
+	// Rows per tile and splits by estimated time: waves of CTAs times the time of one.
+	const int nkb = a.K / TC_BK, tiles = a.N / TN;
+	const int cap = g_tc_force ? std::min(TC_MAX_NR, 64 * g_tc_force) : TC_MAX_NR;
+	const int mt_min = (a.M + cap - 1) / cap;
+	double best = 1e30;
+	int best_splits = 1;
+	for (int mt = mt_min; mt <= mt_min + (g_tc_force ? 0 : 3); ++mt) {
+		const int nr = ((a.M + mt - 1) / mt + 15) & ~15;
+		if ((mt - 1) * nr >= a.M) break;                                 // an empty tile
+		for (int splits = 1; splits <= std::min(TC_MAX_SPLITS, nkb); ++splits) {
+			const int per = splits == 1 ? nkb : ((nkb + splits - 1) / splits + 1) & ~1;      // whole stages
+			if ((splits - 1) * per >= nkb) continue;                     // an empty split
+			if (g_tc_splitk > 0 ? splits != g_tc_splitk : splits > 1 && per < 4) continue;
+			const int n = slots_of(splits);
+			if (n <= 0) continue;
+			const long long ctas = (long long)mt * tiles * splits;
+			const double t = (double)((ctas + n - 1) / n) * tc_cta_us(nr, splits, per);
+			if (t < best) {
+				best = t;
+				best_splits = splits;
+				p.nr = nr;
+				p.kb_per_split = per;
+			}
+		}
+	}
+	if (best >= 1e30) {          // a forced split that is not possible: none
+		p.nr = ((a.M + mt_min - 1) / mt_min + 15) & ~15;
+		p.kb_per_split = nkb;
+	}
+	return p.nr <= TC_PAIR_NR ? tc_go<EPI, 2>(p, best_splits, dev, stream) : tc_go<EPI, 1>(p, best_splits, dev, stream);
 }
 
 int tc_launch(const TcArgs &a, int epi, void *workspace, size_t ws_bytes, cudaStream_t stream) {
 	if (a.perm) return GPTQ_ERR_UNSUPPORTED;
 	if (!workspace || ws_bytes < 16384) return GPTQ_ERR_WORKSPACE;
 	if (a.ldx % 8 != 0) return GPTQ_ERR_ALIGN;
-	alignas(64) CUtensorMap tmx;
-	if (int rc = x_tensor_map(a.x, a.M, a.K, a.ldx, &tmx)) return rc;
-	TcParams p;
+	TcParams p = {};
 	p.a = a;
-	p.epi = epi;
 	p.status = reinterpret_cast<int *>(workspace) + (16384 / 4 - 1);
-	p.kb_per_split = a.K / TC_BK;
-	p.partial = nullptr;
-	// Tile choice: estimated time = waves * (rows * columns of a tile) / relative speed of the configuration
-	// (measured per busy SM: 128 x 128 tiles 1.0, 128 x 256 tiles 1.7, 256-row tiles 2.5).
-	int dev = 0, sms = 148;
-	if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	auto cost = [&](int bm, int bn, double speed) {
-		if (a.N % bn != 0) return 1e30;
-		const long long tiles = (long long)(a.N / bn) * ((a.M + bm - 1) / bm);
-		const long long waves = (tiles + sms - 1) / sms;
-		return (double)waves * bm * bn / speed;
-	};
-	if (epi == TC_EPI_SILU) {
-		const bool tall = g_tc_force ? (g_tc_force >= 3) : (cost(256, 128, 1.5) < cost(128, 128, 1.0));
-		return tall ? tc_launch_inst<2, TC_EPI_SILU, 128, 2>(tmx, p, stream) : tc_launch_inst<2, TC_EPI_SILU, 128, 1>(tmx, p, stream);
-	}
-	// configurations: 0 = 128 x 128, 1 = 128 x 256, 2 = 256 x 256, 3 = 256 x 128
-	int pick = 0;
-	if (epi == TC_EPI_PLAIN) {
-		// Plain epilogue: tile configuration AND split-K by estimated time.  Measured on B200 (M = 512 and 1024,
-		// N = 4096, K = 4096 and 11008): a CTA needs t_kb microseconds per K-block of 64 whatever the number of CTAs
-		// (0.66 for 128 x 128 tiles, 0.73 for 128 x 256, 0.91 for 256 x 256, 0.82 for 256 x 128) plus about 2.5 us
-		// to start and drain; split-K costs about 6 us (second launch, strided fp32 stores) plus the partial sums
-		// written and read back at about 4 TB/s.  Short prompts with a long K gain most (M = 512, 11008 -> 4096:
-		// 102 -> 62 us); M = 512, 4096 -> 4096 gains 10 %.
-		const int bms[4] = {128, 128, 256, 256}, bns[4] = {128, 256, 256, 128};
-		const double t_kbs[4] = {0.66, 0.73, 0.91, 0.82};
-		const int nkb = a.K / TC_BK;
-		const bool room = ws_bytes >= 16384 + (size_t)TC_MAX_SPLITK * a.M * a.N * 4 && (size_t)TC_MAX_SPLITK * a.M * a.N * 4 <= TC_SPLIT_BYTES;
-		double best = 1e30;
-		int best_sk = 1;
-		for (int i = 0; i < 4; ++i) {
-			if (a.N % bns[i] != 0) continue;
-			if (g_tc_force && i != (((g_tc_force == 2 || g_tc_force == 3) && a.N % 256 != 0) ? 0 : g_tc_force - 1)) continue;
-			const double t_kb = t_kbs[i];
-			const long long tiles = (long long)(a.N / bns[i]) * ((a.M + bms[i] - 1) / bms[i]);
-			for (int sk = 1; sk <= TC_MAX_SPLITK; sk *= 2) {
-				if (sk > 1 && (!room || nkb < sk)) break;
-				if (g_tc_splitk > 0) {
-					if (sk != g_tc_splitk) continue;                 // forced by a test
-				} else if (sk > 1 && nkb / sk < 8) {
-					break;                                           // too few K-blocks per split to amortise the start / drain
-				}
-				const int kbps = (nkb + sk - 1) / sk;
-				const long long waves = (tiles * ((nkb + kbps - 1) / kbps) + sms - 1) / sms;
-				double t = (double)waves * (kbps * t_kb + 2.5);
-				if (sk > 1) t += 6.0 + (double)sk * a.M * a.N * 8.0 / 4.0e6;
-				if (t < best) {
-					best = t;
-					pick = i;
-					best_sk = sk;
-				}
-			}
-		}
-		p.kb_per_split = (nkb + best_sk - 1) / best_sk;
-		p.partial = best_sk > 1 ? reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(workspace) + 16384) : nullptr;
-	} else {
-		const double c[4] = {cost(128, 128, 1.0), cost(128, 256, 1.7), cost(256, 256, 2.5), cost(256, 128, TC_SPEED_256x128)};
-		for (int i = 1; i < 4; ++i)
-			if (c[i] < c[pick]) pick = i;
-		if (g_tc_force) pick = ((g_tc_force == 2 || g_tc_force == 3) && a.N % 256 != 0) ? 0 : g_tc_force - 1;
+	if (epi == TC_EPI_ROPE) {
+		auto even = [](const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 7u) == 0; };
+		p.out8 = even(a.q_out) && even(a.k_out) && even(a.v_out) && ((a.q_stride_m | a.kv_sb | a.kv_st | a.kv_sh | a.kv_sp) & 3) == 0;
 	}
 	switch (epi) {
-		case TC_EPI_PLAIN:
-			return pick == 3 ? tc_launch_inst<1, TC_EPI_PLAIN, 128, 2>(tmx, p, stream)
-				 : pick == 2 ? tc_launch_inst<1, TC_EPI_PLAIN, 256, 2>(tmx, p, stream)
-				 : pick == 1 ? tc_launch_inst<1, TC_EPI_PLAIN, 256, 1>(tmx, p, stream) : tc_launch_inst<1, TC_EPI_PLAIN, 128, 1>(tmx, p, stream);
-		case TC_EPI_ROPE:
-			return pick == 3 ? tc_launch_inst<1, TC_EPI_ROPE, 128, 2>(tmx, p, stream)
-				 : pick == 2 ? tc_launch_inst<1, TC_EPI_ROPE, 256, 2>(tmx, p, stream)
-				 : pick == 1 ? tc_launch_inst<1, TC_EPI_ROPE, 256, 1>(tmx, p, stream) : tc_launch_inst<1, TC_EPI_ROPE, 128, 1>(tmx, p, stream);
+		case TC_EPI_PLAIN: return tc_launch_inst<TC_EPI_PLAIN>(p, stream);
+		case TC_EPI_SILU: return tc_launch_inst<TC_EPI_SILU>(p, stream);
+		case TC_EPI_ROPE: return tc_launch_inst<TC_EPI_ROPE>(p, stream);
 	}
 	return GPTQ_ERR_INVALID;
 }

@@ -660,3 +660,30 @@ def test_prefill_split_k(G, cfg, sk):
 		_lib.lib().gptq_debug_tc_splitk(0)
 	assert O.max_rel_err(y, ref) <= TOL
 	assert _lib.kernel_status() == 0
+
+
+@pytest.mark.parametrize('sk', [1, 3, 8])
+@pytest.mark.parametrize('M,K,gs', [(17, 1984, 64), (33, 1024, -1), (144, 1920, 128), (145, 1984, 64), (256, 1024, 512), (257, 1920, 192)])
+def test_prefill_edges_of_row_tiles_and_splits(G, M, K, gs, sk):
+	"""Rows just below and above a tile of the tensor-core kernel (stages of two K-blocks up to 144 rows, one above; 256 rows per tile),
+	odd numbers of K-blocks, groups that end inside a stage, and clusters of 1, 3 and 8 CTAs, with every epilogue."""
+	from gptq_triton_b200 import _lib
+	H, D, N = 2, 128, 256
+	t, g, u, w = synth(K, N, gs, 1, bias=True), synth(K, N, gs, 2), synth(K, N, gs, 3), synth(K, 3 * H * D, gs, 4)
+	x, res = acts((M, K), seed=5), acts((M, N), seed=6)
+	pos = torch.arange(M).flip(0).unsqueeze(0).contiguous()
+	cos, sin = O.rope_tables(D, 512)
+	c = lambda d: (d['qweight'].cuda(), d['scales'].cuda(), d['qzeros'].cuda())
+	try:
+		_lib.lib().gptq_debug_tc_splitk(sk)
+		y = G.qmatmul(gs, x.cuda(), *c(t), bias=t['bias'].cuda(), residual=res.cuda())
+		h = G.gateup_silu(gs, x.cuda(), *c(g), *c(u))
+		q, k, v = G.qkv_rope(gs, x.view(1, M, K).cuda(), *c(w), cos.cuda(), sin.cuda(), pos.cuda(), H, D)
+		torch.cuda.synchronize()
+	finally:
+		_lib.lib().gptq_debug_tc_splitk(0)
+	assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, bias=t['bias'], residual=res)) <= TOL
+	assert O.max_rel_err(h, O.gateup_silu_r32(x, (g['qweight'], g['qzeros'], g['scales']), (u['qweight'], u['qzeros'], u['scales']), gs)) <= TOL
+	rq, rk, rv = O.qkv_rope_r32(x.view(1, M, K), w['qweight'], w['qzeros'], w['scales'], gs, cos, sin, pos, H, D)
+	assert O.max_rel_err(q.transpose(1, 2), rq) <= TOL and O.max_rel_err(k.transpose(1, 2), rk) <= TOL and O.max_rel_err(v.transpose(1, 2), rv) <= TOL
+	assert _lib.kernel_status() == 0
