@@ -80,6 +80,7 @@ _OPTIONAL = {
 	'gptq_debug_soft_max_splits': (None, [c_int]),
 	'gptq_debug_allow_narrow': (None, [c_int]),
 	'gptq_debug_tc_force': (None, [c_int]),
+	'gptq_debug_dec_min_rows': (None, [c_int]),
 	'gptq_debug_tc_splitk': (None, [c_int]),
 	'gptq_debug_chain_stages': (None, [c_int]),
 }

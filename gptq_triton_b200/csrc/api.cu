@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "attn_decode.cuh"
 #include "qkv_attn.cuh"
+#include "qmm_dec.cuh"
 #include "qmm_skinny.cuh"
 #include "qmm_tc.cuh"
 
@@ -21,6 +22,7 @@ static int g_max_stages2 = 3;    // the same for the two-stream (gate/up) form (
 static int g_max_stages = 4;     // tuning hook: upper bound of the ring depth of the decode kernel
 static int g_soft_max_splits = 8;  // the planner avoids more splits than this (gptq_debug_soft_max_splits)
 static int g_qa_stages = 2;       // ring depth of the attention-block kernel (gptq_debug_qa_stages); 7B step, gate/up at 3 stages: 4 / 3 / 2 stages 589 / 596 / 600 tokens/s at 2.1 k context, 453 / 457 / 457 at 8 k, 660 / 676 / 681 at 300
+static int g_dec_min_rows = 0;    // tests: rows from which a decode call runs on the tensor-memory kernel (gptq_debug_dec_min_rows; 17: never), 0 = by size
 static int g_pdl = 1;             // programmatic dependent launch for the decode-step kernels (+3 % on the decode step)
 
 bool pdl_enabled() { return g_pdl != 0; }      // for the launchers in the other files
@@ -235,6 +237,15 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 	grid = dim3(tiles, p.splitk, 1);
 }
 
+// Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one.  Its time hardly depends on the rows, its start and end cost
+// about 4 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor memory / this
+// kernel: 4096 -> 4096 (8 MB) M = 4 8.5 / 7.4, M = 8 8.5 / 10.1; 11008 -> 4096 (23 MB) M = 4 11.7 / 11.2, M = 8 11.9 / 13.9;
+// 22016 -> 8192 (90 MB) M = 1 25.9 / 23.8, M = 4 26.1 / 28.8, M = 16 28.2 / 55.3; gate/up 8192 -> 2 x 22016 (180 MB) M = 1 48.5 / 48.0, M = 16 61 / 110.
+static int dec_min_rows(int K, int N, int nstream) {
+	const double mb = (double)K * N * nstream / 2e6;
+	return mb >= 64 ? 4 : mb >= 20 ? 6 : 7;
+}
+
 // Narrow geometry (one 32-column strip and the whole of K per CTA, no split-K): worth it when
 // N / 32 CTAs fill most of the chip in one wave and the x rows of the whole K fit in shared memory.
 static int g_allow_narrow = 0;      // opt-in (gptq_debug_allow_narrow): measured slower than the tiled split-K form
@@ -316,7 +327,7 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 		p.ws_words = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(workspace) + words_offset(need));
 	if (p.perm) {
 		// act-order: x[:, perm] once, into the workspace behind the partial sums (or at the offset the caller planned)
-		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(words_offset(need) + words_bytes(p.M, need));
+		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(std::max(words_offset(need) + words_bytes(p.M, need), dec_ws_bytes(p.M)));
 		if (ws_bytes < off + gather_bytes(p.M, p.K)) return GPTQ_ERR_WORKSPACE;
 		__half *xp = reinterpret_cast<__half *>(reinterpret_cast<unsigned char *>(workspace) + off);
 		const dim3 gg((unsigned)((p.K / 8 + 255) / 256), (unsigned)p.M, 1);
@@ -324,6 +335,19 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 		p.x = xp;
 		p.ldx = p.K;
 		p.perm = nullptr;
+	}
+	if (gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow && p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) &&
+		ws_bytes >= dec_ws_bytes(p.M)) {
+		DecArgs a = {};
+		a.x = p.x; a.ldx = p.ldx;
+		a.qw0 = qw0; a.qw1 = qw1; a.qz0 = p.qz0; a.qz1 = p.qz1; a.sc0 = p.sc0; a.sc1 = p.sc1;
+		a.M = p.M; a.K = p.K; a.N = p.N; a.groupsize = p.groupsize;
+		a.bias = p.bias; a.residual = p.residual; a.ldr = p.ldr; a.y = p.y; a.ldy = p.ldy; a.ss_out = p.ss_out;
+		a.rms_w = p.rms_w; a.ss_in = p.ss_in; a.ss_tiles = p.ss_tiles; a.rms_eps = p.rms_eps;
+		a.cos_t = p.cos_t; a.sin_t = p.sin_t; a.pos = p.pos; a.q_out = p.q_out; a.k_out = p.k_out; a.v_out = p.v_out;
+		a.q_stride_m = p.q_stride_m; a.kv_sb = p.kv_sb; a.kv_st = p.kv_st; a.kv_sh = p.kv_sh; a.kv_sp = p.kv_sp;
+		a.tokens_per_batch = p.tokens_per_batch; a.hidden = p.hidden; a.max_pos = p.max_pos;
+		return dec_launch(a, EPI == EPI_SILU ? DEC_EPI_SILU : EPI == EPI_ROPE ? DEC_EPI_ROPE : DEC_EPI_PLAIN, workspace, ws_bytes, stream);
 	}
 	p.ws_ticket = reinterpret_cast<int *>(workspace);
 	p.ws_partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(workspace) + SK_TICKET_BYTES);
@@ -427,6 +451,7 @@ int gptq_last_cuda_error(void) { return g_last_cuda_error; }
 void gptq_debug_force_splitk(int splitk) { g_force_splitk = splitk; }
 void gptq_debug_max_stages(int n) { g_max_stages = std::max(2, std::min(n, 8)); }
 void gptq_debug_max_stages2(int n) { g_max_stages2 = std::max(2, std::min(n, 8)); }
+void gptq_debug_dec_min_rows(int n) { g_dec_min_rows = n; }
 void gptq_debug_set_pdl(int on) { g_pdl = on ? 1 : 0; }
 void gptq_debug_qa_stages(int n) { g_qa_stages = n; }
 void gptq_debug_soft_max_splits(int n) { g_soft_max_splits = n; }
@@ -434,7 +459,7 @@ void gptq_debug_allow_narrow(int on) { g_allow_narrow = on ? 1 : 0; }
 size_t gptq_workspace_bytes(int M, int K, int N) {
 	if (M <= 0 || N <= 0) return SK_TICKET_BYTES;
 	const size_t base = skinny_ws_bytes(M, N, 2);
-	return std::max(gather_offset(words_offset(base) + words_bytes(M, base)) + gather_bytes(M, std::max(K, 0)), tc_ws_bytes(M, N));
+	return std::max(gather_offset(std::max(words_offset(base) + words_bytes(M, base), dec_ws_bytes(M))) + gather_bytes(M, std::max(K, 0)), tc_ws_bytes(M, N));
 }
 
 struct ArArgs {

@@ -8,11 +8,11 @@
 //   - The N of an MMA is any multiple of 16 up to 256, so a tile holds exactly the rows that there are: 40 rows cost 48, not 128.
 // A CTA computes 128 columns (64 gate + 64 up columns for the fused MLP) x nr rows; K advances in blocks of 64.
 //
-//   warp 0      packed weights (8 words x 128 columns per K-block), scales and zeros by TMA / bulk copies into a deep ring
+//   warp 0      packed weights (8 words x 128 columns per K-block) by TMA into a deep ring; warp 3 their scales and zeros
 //   warp 1      X tile [nr x 64] fp16, K-major, 128-byte swizzle
 //   warp 2      MMA issuer: tcgen05.mma.cta_group::1.kind::f16, A from tensor memory, M = 128, N = nr, K = 16; one wait and one
 //               commit per stage of one or two K-blocks
-//   warp 3      owns the tensor-memory allocation (nr columns of accumulators, 4 to 8 stages of 32 or 64 columns of weights)
+//   warp 3      also owns the tensor-memory allocation (nr columns of accumulators, 4 to 8 stages of 32 or 64 columns of weights)
 //   warps 4-19  dequantise, four groups of four warps, group j serving the stages j, j + 4, ...: 8 packed words of a column
 //               become 64 fp16 weights (q - zero) * scale with ONE rounding each, the weights of the dequantise-then-matmul path
 // Afterwards the accumulators are turned through shared memory into an fp32 tile [row][128] and all warps run the epilogue:

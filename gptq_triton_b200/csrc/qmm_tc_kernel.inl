@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 			mbar_init(bar_empty + 8 * s, 1);
 		}
 		for (int s = 0; s < PW; ++s) {
-			mbar_init(bar_full_w + 8 * s, 1);
+			mbar_init(bar_full_w + 8 * s, 2);                 // words; scales and zeros
 			mbar_init(bar_empty_w + 8 * s, 4);                // one arrival per warp of the consuming group
 		}
 		mbar_init(bar_acc, 1);
@@ -67,42 +67,56 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 	// One lane of the three serial roles does the work, but the whole warp walks the loop: its addresses and descriptors are then
 	// warp-uniform.  With a loop for lane 0 alone the issuer needed 0.40 us per K-block and was the bound of every short prompt
 	// (M = 40, 4096 -> 12288: 28.3 us; uniform: 16.4 us; with two K-blocks per stage 13.9 us).
-	if (warp == 0) {
-		// ---------------- packed weights, scales and zeros (weights depend on no earlier kernel) ----------------
-		const int gk = a.groupsize / TC_BK, nz = a.N >> 3, g_last = a.K / a.groupsize - 1;
-		int g = kb0 / gk, left = gk - (kb0 - g * gk), s = 0;          // group of the stage's first block, blocks left in it
-		uint32_t ph = 1;
+	if (warp == 0 || warp == 3) {
+		// ---------------- packed weights (warp 0), scales and zeros (warp 3); they depend on no earlier kernel ----------------
+		const int gk = a.groupsize / TC_BK, nz = a.N >> 3, g0 = kb0 / gk;
+		int left = gk - (kb0 - g0 * gk), s = 0, row = kb0 * 8, groups = a.K / a.groupsize - g0;      // blocks left in the group, groups left
+		const __half *sc0 = a.sc0 + (size_t)g0 * a.N + n0, *sc1 = PAIR ? a.sc1 + (size_t)g0 * a.N + n0 : nullptr;
+		const int32_t *qz0 = a.qz0 + (size_t)g0 * nz + (n0 >> 3), *qz1 = PAIR ? a.qz1 + (size_t)g0 * nz + (n0 >> 3) : nullptr;
+		uint32_t ph = 1, dst = sW, bar = bar_full_w;
 		const bool one = tc_elect();
 		for (int i = 0; i < n; ++i) {
-			if (!tc_wait(bar_empty_w + 8 * s, ph, s_abort)) { fail(); settle(); break; }
+			if (!tc_wait(bar + (bar_empty_w - bar_full_w), ph, s_abort)) { fail(); settle(); break; }
 			if (one) {
-				const uint32_t dst = sW + s * W_STAGE, bar = bar_full_w + 8 * s;
-				const int kw = (kb0 + KP * i) * 8;
-				auto group = [&](int h, int gg) {
-					const uint32_t sc = dst + W_SC + h * 256, qz = dst + W_QZ + h * 64;
-					const size_t so = (size_t)gg * a.N + n0, zo = (size_t)gg * nz + (n0 >> 3);
-					tc_bulk_load(sc, a.sc0 + so, TN * 2, bar);
-					tc_bulk_load(qz, a.qz0 + zo, TN / 2, bar);
-					if (PAIR) {
-						tc_bulk_load(sc + 128, a.sc1 + so, TN * 2, bar);
-						tc_bulk_load(qz + 32, a.qz1 + zo, TN / 2, bar);
-					}
-				};
-				mbar_arrive_expect_tx(bar, W_SC + sets * 320);
-				tma_load_2d(dst, &tmw0, n0, kw, bar);              // (packed rows behind K read as zero)
-				if (PAIR) tma_load_2d(dst + W_SC / 2, &tmw1, n0, kw, bar);
-				group(0, g);
-				if (KP == 2 && sets == 2) group(1, left > 1 ? g : min(g + 1, g_last));
+				if (warp == 0) {
+					mbar_arrive_expect_tx(bar, W_SC);
+					tma_load_2d(dst, &tmw0, n0, row, bar);             // (packed rows behind K read as zero)
+					if (PAIR) tma_load_2d(dst + W_SC / 2, &tmw1, n0, row, bar);
+				} else {
+					auto group = [&](int h, size_t more) {
+						const uint32_t sc = dst + W_SC + h * 256, qz = dst + W_QZ + h * 64;
+						tc_bulk_load(sc, sc0 + more * a.N, TN * 2, bar);
+						tc_bulk_load(qz, qz0 + more * nz, TN / 2, bar);
+						if (PAIR) {
+							tc_bulk_load(sc + 128, sc1 + more * a.N, TN * 2, bar);
+							tc_bulk_load(qz + 32, qz1 + more * nz, TN / 2, bar);
+						}
+					};
+					mbar_arrive_expect_tx(bar, sets * 320);
+					group(0, 0);
+					if (KP == 2 && sets == 2) group(1, left == 1 && groups > 1 ? 1 : 0);
+				}
 			}
+			__syncwarp();
+			row += 8 * KP;
 #pragma unroll
 			for (int h = 0; h < KP; ++h)
 				if (--left == 0) {
-					++g;
 					left = gk;
+					--groups;
+					sc0 += a.N;
+					qz0 += nz;
+					if (PAIR) {
+						sc1 += a.N;
+						qz1 += nz;
+					}
 				}
-			__syncwarp();
+			dst += W_STAGE;
+			bar += 8;
 			if (++s == PW) {
 				s = 0;
+				dst = sW;
+				bar = bar_full_w;
 				ph ^= 1;
 			}
 		}

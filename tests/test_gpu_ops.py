@@ -687,3 +687,40 @@ def test_prefill_edges_of_row_tiles_and_splits(G, M, K, gs, sk):
 	rq, rk, rv = O.qkv_rope_r32(x.view(1, M, K), w['qweight'], w['qzeros'], w['scales'], gs, cos, sin, pos, H, D)
 	assert O.max_rel_err(q.transpose(1, 2), rq) <= TOL and O.max_rel_err(k.transpose(1, 2), rk) <= TOL and O.max_rel_err(v.transpose(1, 2), rv) <= TOL
 	assert _lib.kernel_status() == 0
+
+
+@pytest.mark.parametrize('M', [1, 7, 8, 9, 16])
+@pytest.mark.parametrize('K,gs,N,act', [(128, -1, 128, False), (1024, 256, 256, True), (4096, 128, 384, False), (2560, 128, 2176, True)])
+def test_decode_tensor_memory_kernel(G, K, gs, N, act, M):
+	"""The decode kernel that keeps weights in tensor memory, forced for every number of rows: one tile of one K-unit, tiles cut by many
+	CTAs, more tiles than CTAs have units, gathered x; every epilogue against the oracle, the folded norm and the sums of squares too."""
+	from gptq_triton_b200 import _lib
+	H, D = 1, 128
+	t, g, u, w = synth(K, N, gs, 1, bias=True, act_order=act), synth(K, N, gs, 2), synth(K, N, gs, 3), synth(K, 3 * H * D, gs, 4)
+	x, res = acts((M, K), seed=5), acts((M, N), seed=6)
+	pos = torch.arange(M).flip(0).unsqueeze(0).contiguous()
+	cos, sin = O.rope_tables(D, 64)
+	c = lambda d: (d['qweight'].cuda(), d['scales'].cuda(), d['qzeros'].cuda())
+	layer = G.QuantLinear(4, gs, K, N, True)
+	layer.qweight, layer.qzeros, layer.scales, layer.bias = t['qweight'], t['qzeros'], t['scales'], t['bias']
+	layer.set_g_idx(t['g_idx'] if act else None)
+	layer = layer.cuda()
+	ss = torch.zeros((M, N // 32), dtype=torch.float32, device='cuda')
+	norm_w = (1 + 0.1 * acts((1, K), seed=7).view(-1)).half()
+	xn = (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-6) * norm_w.float()).half()
+	ss_in = x.float().pow(2).view(M, K // 32, 32).sum(-1).contiguous().cuda()
+	try:
+		_lib.lib().gptq_debug_dec_min_rows(1)
+		y = layer(x.cuda(), residual=res.cuda(), sumsq_out=ss)
+		h = G.gateup_silu(gs, x.cuda(), *c(g), *c(u), rms_weight=norm_w.cuda(), rms_eps=1e-6, sumsq_in=ss_in)
+		q, k, v = G.qkv_rope(gs, x.view(1, M, K).cuda(), *c(w), cos.cuda(), sin.cuda(), pos.cuda(), H, D)
+		torch.cuda.synchronize()
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	gi = dict(g_idx=t['g_idx']) if act else {}
+	assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, bias=t['bias'], residual=res, **gi)) <= TOL
+	assert torch.allclose(ss, y.float().pow(2).view(M, N // 32, 32).sum(-1), rtol=1e-5)          # 32 fp32 terms in another order
+	assert O.max_rel_err(h, O.gateup_silu_r32(xn, (g['qweight'], g['qzeros'], g['scales']), (u['qweight'], u['qzeros'], u['scales']), gs)) <= TOL
+	rq, rk, rv = O.qkv_rope_r32(x.view(1, M, K), w['qweight'], w['qzeros'], w['scales'], gs, cos, sin, pos, H, D)
+	assert O.max_rel_err(q.transpose(1, 2), rq) <= TOL and O.max_rel_err(k.transpose(1, 2), rk) <= TOL and O.max_rel_err(v.transpose(1, 2), rv) <= TOL
+	assert _lib.kernel_status() == 0
