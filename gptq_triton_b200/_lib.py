@@ -6,6 +6,7 @@ raised.  The library is built in-tree by `python -m gptq_triton_b200.build`.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
@@ -129,12 +130,21 @@ def check(code: int, what: str):
 		raise err(f'{what}: {msg}{extra}')
 
 
+# Addresses and streams go to ctypes as plain integers and the stream is asked for without building a Stream object: a call of the
+# smallest layer is bound by the host (o_proj of a 7B layer for one token: 27 us a call, 6 of them on the GPU).
 def ptr(t: Optional[torch.Tensor]):
-	return None if t is None else c_void_p(t.data_ptr())
+	return None if t is None else t.data_ptr()
 
 
-def stream_ptr(device) -> c_void_p:
-	return c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def stream_ptr(device) -> int:
+	return _raw_stream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+def _raw_stream(index: int) -> int:
+	return torch.cuda.current_stream(index).cuda_stream
+
+
+_raw_stream = getattr(torch._C, '_cuda_getCurrentRawStream', _raw_stream)
 
 
 def require_cuda(*tensors):
@@ -148,10 +158,15 @@ def require_cuda(*tensors):
 _workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 
 
+@functools.lru_cache(maxsize=4096)
+def _workspace_bytes(M: int, K: int, N: int) -> int:          # (depends on the sizes alone)
+	return lib().gptq_workspace_bytes(M, K, N)
+
+
 def workspace(device: torch.device, M: int, K: int, N: int, min_bytes: int = 0) -> torch.Tensor:
-	need = max(lib().gptq_workspace_bytes(M, K, N), min_bytes)
-	key = (device.index if device.index is not None else torch.cuda.current_device(),
-		   torch.cuda.current_stream(device).cuda_stream)
+	need = max(_workspace_bytes(M, K, N), min_bytes)
+	index = device.index if device.index is not None else torch.cuda.current_device()
+	key = (index, _raw_stream(index))
 	ws = _workspaces.get(key)
 	if ws is None or ws.numel() < need:
 		if ws is not None:

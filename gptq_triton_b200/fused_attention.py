@@ -76,7 +76,7 @@ def qkv_rope(groupsize: int, a: torch.Tensor, qweight, scales, qzeros, cos, sin,
 	if rms_weight is not None:
 		a = rmsnorm(a, rms_weight, rms_eps)          # the norm runs as its own kernel
 	if M > DECODE_MAX_M and perm is not None and prefill_kernel_available(M, K, 3 * hidden, groupsize):
-		a = a.view(M, K)[:, perm.long()].contiguous().view(b, t, K)
+		a = a.view(M, K).index_select(1, perm).view(b, t, K)
 		perm = None
 	if M > DECODE_MAX_M and not prefill_kernel_available(M, K, 3 * hidden, groupsize):
 		y = dequant_matmul(a.view(M, K), groupsize, qweight, scales, qzeros, None, perm).float().view(b, t, 3, n_heads, head_dim)

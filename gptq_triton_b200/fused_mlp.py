@@ -53,12 +53,12 @@ def gateup_silu(groupsize: int, a: torch.Tensor, gate_qweight, gate_scales, gate
 	_lib.require_cuda(a, gate_qweight, gate_scales, gate_qzeros, up_qweight, up_scales, up_qzeros, g_idx, perm)
 	if a.dtype != torch.float16:
 		raise TypeError('A must be float16')
-	x = a.view(-1, a.shape[-1])
-	M, K = x.shape
-	N = gate_qweight.shape[1]
-	c = torch.empty((M, N), device=a.device, dtype=torch.float16)
+	K, N = a.shape[-1], gate_qweight.shape[1]
+	M = a.numel() // K
+	c = torch.empty(a.shape[:-1] + (N,), device=a.device, dtype=torch.float16)
 	if M == 0:
-		return c.view(a.shape[:-1] + (N,))
+		return c
+	x = a
 	from .quant_linear import DECODE_MAX_M, dequant_matmul, prefill_kernel_available, rms_fusable
 	if rms_weight is not None and sumsq_in is not None and rms_fusable(M, K, g_idx, perm):
 		assert sumsq_in.dtype == torch.float32 and sumsq_in.is_contiguous() and sumsq_in.numel() >= M * (K // 32)
@@ -69,26 +69,27 @@ def gateup_silu(groupsize: int, a: torch.Tensor, gate_qweight, gate_scales, gate
 			_lib.ptr(c), M, K, N, groupsize, K, N, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device),
 			_lib.ptr(rms_weight), _lib.ptr(sumsq_in), K // 32, float(rms_eps))
 		_lib.check(rc, 'gptq_gateup_silu_rms')
-		return c.view(a.shape[:-1] + (N,))
+		return c
 	if rms_weight is not None:
 		from .fused_attention import rmsnorm
-		x = rmsnorm(x.contiguous(), rms_weight, rms_eps)
+		x = rmsnorm(x, rms_weight, rms_eps)
 		rms_weight = None
-	if M > DECODE_MAX_M and perm is not None and g_idx is None and prefill_kernel_available(M, K, N, groupsize):
-		x = x[:, perm.long()].contiguous()
-		perm = None
-	if M > DECODE_MAX_M and (g_idx is not None or not prefill_kernel_available(M, K, N, groupsize)):
-		g = dequant_matmul(x, groupsize, gate_qweight, gate_scales, gate_qzeros, g_idx, perm).float()
-		u = dequant_matmul(x, groupsize, up_qweight, up_scales, up_qzeros, g_idx, perm).float()
-		c = (torch.nn.functional.silu(g) * u).half()
-		return c.view(a.shape[:-1] + (N,))
+	if M > DECODE_MAX_M:
+		if g_idx is not None or not prefill_kernel_available(M, K, N, groupsize):
+			x = x.view(M, K)
+			g = dequant_matmul(x, groupsize, gate_qweight, gate_scales, gate_qzeros, g_idx, perm).float()
+			u = dequant_matmul(x, groupsize, up_qweight, up_scales, up_qzeros, g_idx, perm).float()
+			return (torch.nn.functional.silu(g) * u).half().view(a.shape[:-1] + (N,))
+		if perm is not None:
+			x = x.view(M, K).index_select(1, perm)
+			perm = None
 	ws = _lib.workspace(a.device, M, K, N)
 	rc = _lib.lib().gptq_gateup_silu(
 		_lib.ptr(x), _lib.ptr(gate_qweight), _lib.ptr(gate_qzeros), _lib.ptr(gate_scales),
 		_lib.ptr(up_qweight), _lib.ptr(up_qzeros), _lib.ptr(up_scales), _lib.ptr(g_idx), _lib.ptr(perm),
 		_lib.ptr(c), M, K, N, groupsize, K, N, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device))
 	_lib.check(rc, 'gptq_gateup_silu')
-	return c.view(a.shape[:-1] + (N,))
+	return c
 
 
 def triton_llama_mlp_4(groupsize: int, a: torch.FloatTensor, gate_qweight: torch.IntTensor, gate_scales: torch.FloatTensor,

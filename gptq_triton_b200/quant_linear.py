@@ -105,26 +105,25 @@ def qmatmul(groupsize: int, a: torch.Tensor, qweight: torch.Tensor, scales: torc
 	_lib.require_cuda(a, qweight, scales, qzeros, bias, g_idx, perm, residual)
 	if a.dtype != torch.float16:
 		raise TypeError('A must be float16')
-	x = a.view(-1, a.shape[-1])
-	M, K = x.shape
-	N = qweight.shape[1]
-	c = torch.empty((M, N), device=a.device, dtype=torch.float16)
+	K, N = a.shape[-1], qweight.shape[1]
+	M = a.numel() // K
+	c = torch.empty(a.shape[:-1] + (N,), device=a.device, dtype=torch.float16)
 	if M == 0:
-		return c.view(a.shape[:-1] + (N,))
-	res = None
+		return c
+	x, res = a, residual
 	if residual is not None:
 		assert residual.is_contiguous() and residual.numel() == M * N
-		res = residual.view(M, N)
-	if M > DECODE_MAX_M and perm is not None and g_idx is None and prefill_kernel_available(M, K, N, groupsize):
-		x = x[:, perm.long()].contiguous()      # the tensor-core kernel reads x through TMA: gather once up front
-		perm = None
-	if M > DECODE_MAX_M and (g_idx is not None or not prefill_kernel_available(M, K, N, groupsize)):
-		c = dequant_matmul(x, groupsize, qweight, scales, qzeros, g_idx, perm)
-		if bias is not None:
-			c = c + bias
-		if res is not None:
-			c = c + res
-		return c.view(a.shape[:-1] + (N,))
+	if M > DECODE_MAX_M:
+		if g_idx is not None or not prefill_kernel_available(M, K, N, groupsize):
+			c = dequant_matmul(a.view(M, K), groupsize, qweight, scales, qzeros, g_idx, perm)
+			if bias is not None:
+				c = c + bias
+			if res is not None:
+				c = c + res.view(M, N)
+			return c.view(a.shape[:-1] + (N,))
+		if perm is not None:
+			x = a.view(M, K).index_select(1, perm)      # the tensor-core kernel reads x through TMA: gather once up front
+			perm = None
 	ws = _lib.workspace(a.device, M, K, N)
 	if ar is not None:
 		if sumsq_out is not None:
@@ -135,7 +134,7 @@ def qmatmul(groupsize: int, a: torch.Tensor, qweight: torch.Tensor, scales: torc
 			_lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device), _lib.ptr(sumsq_out),
 			ar.world, ar.rank, ar.partials, ar.flags)
 		_lib.check(rc, 'gptq_qmatmul_ar')
-		return c.view(a.shape[:-1] + (N,))
+		return c
 	if sumsq_out is not None:
 		assert sumsq_out.dtype == torch.float32 and sumsq_out.is_contiguous() and sumsq_out.numel() >= M * (N // 32)
 		rc = _lib.lib().gptq_qmatmul_sumsq(
@@ -143,13 +142,13 @@ def qmatmul(groupsize: int, a: torch.Tensor, qweight: torch.Tensor, scales: torc
 			_lib.ptr(bias), _lib.ptr(res), N, _lib.ptr(c), M, K, N, groupsize, K, N,
 			_lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device), _lib.ptr(sumsq_out))
 		_lib.check(rc, 'gptq_qmatmul_sumsq')
-		return c.view(a.shape[:-1] + (N,))
+		return c
 	rc = _lib.lib().gptq_qmatmul(
 		_lib.ptr(x), _lib.ptr(qweight), _lib.ptr(qzeros), _lib.ptr(scales), _lib.ptr(g_idx), _lib.ptr(perm),
 		_lib.ptr(bias), _lib.ptr(res), N, _lib.ptr(c), M, K, N, groupsize, K, N,
 		_lib.ptr(ws), ws.numel(), _lib.stream_ptr(a.device))
 	_lib.check(rc, 'gptq_qmatmul')
-	return c.view(a.shape[:-1] + (N,))
+	return c
 
 
 def rms_fusable(M: int, N_producer: int, g_idx, perm) -> bool:
