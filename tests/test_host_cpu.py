@@ -147,3 +147,20 @@ def test_bench_reference_arm_prints_one_json_line():
 	assert line['impl'] == 'reference' and line['unit'] == 'tokens/s' and line['value'] > 0
 	assert line['cpu_baseline']['kind'] == 'port' and line['cpu_baseline']['cores'] >= 1 and line['cpu_baseline']['factor'] == 32
 	assert line['e2e'] == {'value': line['value'], 'unit': 'tokens/s', 'h2d_bytes_per_step': 0, 'd2h_bytes_per_step': 0}
+
+
+@pytest.mark.parametrize('b,t,S', [(1, 200, 265), (3, 200, 265), (1, 256, 264), (2, 3, 5)])
+def test_aligned_mask_has_the_same_values(b, t, S):
+	"""Rows of a large additive mask start on 16 bytes afterwards; values, shape and the sharing over the batch stay, small masks and
+	masks of truth values are passed on."""
+	from gptq_triton_b200.fused_attention import aligned_mask
+	mask = torch.randn(1, 1, t, S).half().expand(b, 1, t, S)
+	out = aligned_mask(mask)
+	assert out.shape == mask.shape and torch.equal(out, mask)
+	if t * S < 1 << 15:
+		assert out is mask
+	else:
+		assert out.stride(-1) == 1 and out.stride(-2) % 8 == 0 and (b == 1 or out.stride(0) == 0)
+	own = torch.randn(b, 1, t, S).half().transpose(-1, -2).contiguous().transpose(-1, -2)          # columns first, one per sequence
+	assert torch.equal(aligned_mask(own), own)
+	assert aligned_mask(None) is None and aligned_mask(mask > 0) .dtype == torch.bool
