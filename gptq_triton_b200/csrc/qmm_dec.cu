@@ -261,6 +261,9 @@ __device__ __noinline__ void dec_stage_x(const DecParams &p, int xw, int lane, u
 	};
 	const int u = lane & 15, r0 = lane >> 4;
 	pdl_wait();
+	// behind the wait: what ran before this kernel is complete when its successor starts; not at all when it stores several cache rows of a
+	// sequence (see common.cuh)
+	if (EPI != DEC_EPI_ROPE || a.tokens_per_batch == 1) pdl_trigger();
 	const bool rms = EPI != DEC_EPI_PLAIN && a.rms_w != nullptr;
 	if (rms) {
 		// 1 / rms of every row from the per-tile sums the producing kernel left (fixed order)
@@ -381,7 +384,6 @@ __global__ void __launch_bounds__(DC_THREADS, 1) dec_kernel(const __grid_constan
 	__syncthreads();
 	tc_fence_after();
 	const uint32_t tmem_a = *s_tmem, tmem_d = tmem_a + DC_STAGES * 64;
-	pdl_trigger();
 
 	auto fail = [&](int code) {
 		*s_abort = 1;

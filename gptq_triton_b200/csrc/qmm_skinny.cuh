@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(KW == 8 ? 256 : KW * 128, KW == 8 ? 2 : 4 / KW
 		// One copy of the staging code (real loops; the first pass issues its loads before the
 		// weight prefetch).  Straight-line code that runs once costs instruction fetch, and this
 		// prologue used to be more than half of the kernel's code.
-		pdl_trigger();
+		if (EPI != EPI_ROPE || p.tokens_per_batch == 1) pdl_trigger();      // several cache rows of a sequence: not early (see common.cuh)
 		const int x_passes = (p.M * u_blocks + XB - 1) / XB;
 		const int n_it = max(max(1, x_passes), (n_strip + NT * SB - 1) / (NT * SB));
 		int xr = 0, xub = 0;                                 // first (row, unit block) item of the current x pass

@@ -28,6 +28,11 @@
 //   M = 512   4096 -> 4096   17.0 (36.0)   11008 -> 4096  36.3 (55.8)   gate/up 4096 -> 2 x 11008   86 (132)
 //   M = 2048  4096 -> 4096   53.2 (58.0)   11008 -> 4096   134 (145)    gate/up 4096 -> 2 x 11008  296 (332)
 //
+// It keeps its place in the stream in both directions: it stores many cache rows and may be the first reader of new weights, so it reads nothing
+// ahead of its dependency wait and never triggers its successor (see pdl_trigger in common.cuh).  As a dependent launch it still has its
+// barriers, tensor memory and launch latency behind it when the kernel in front ends: a layer of 512 rows 4096 -> 4096 takes 19.1 us per call,
+// 20.5 as a plain launch; with weights ahead of the wait and an early trigger, which let attention read unfinished cache rows, it took 18.5.
+//
 // Every mbarrier wait is bounded; a wait that runs out sets a status word and the kernel unwinds (tensor memory is still released).
 #include <algorithm>
 #include <atomic>

@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 	__syncthreads();
 	tc_fence_after();
 	const uint32_t tmem = *s_tmem, tmem_a = tmem + TC_TMEM_COLS - S * (KP * TC_BK / 2);      // accumulators in front
-	pdl_trigger();
+
+	pdl_wait();          // nothing of earlier kernels, weights included, has been touched so far
 
 	auto fail = [&]() {
 		*s_abort = 1;
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 	// warp-uniform.  With a loop for lane 0 alone the issuer needed 0.40 us per K-block and was the bound of every short prompt
 	// (M = 40, 4096 -> 12288: 28.3 us; uniform: 16.4 us; with two K-blocks per stage 13.9 us).
 	if (warp == 0 || warp == 3) {
-		// ---------------- packed weights (warp 0), scales and zeros (warp 3); they depend on no earlier kernel ----------------
+		// ---------------- packed weights (warp 0), scales and zeros (warp 3) ----------------
 		const int gk = a.groupsize / TC_BK, nz = a.N >> 3, g0 = kb0 / gk;
 		int left = gk - (kb0 - g0 * gk), s = 0, row = kb0 * 8, groups = a.K / a.groupsize - g0;      // blocks left in the group, groups left
 		const __half *sc0 = a.sc0 + (size_t)g0 * a.N + n0, *sc1 = PAIR ? a.sc1 + (size_t)g0 * a.N + n0 : nullptr;
@@ -122,7 +123,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 		}
 	} else if (warp == 1) {
 		// ---------------- X tiles (rows beyond M and columns beyond K are filled with zeros by the copy) ----------------
-		pdl_wait();
 		int s = 0;
 		uint32_t ph = 1;
 		const bool one = tc_elect();
@@ -266,7 +266,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 		tc_fence_after();
 		tmem_dealloc(tmem, TC_TMEM_COLS);
 	}
-	pdl_wait();
 
 	// ---------------- epilogue: the CTAs of a split share the rows; partial tiles are summed in split order ----------------
 	const int live = min(p.nr, a.M - m0);

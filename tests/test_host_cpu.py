@@ -164,3 +164,18 @@ def test_aligned_mask_has_the_same_values(b, t, S):
 	own = torch.randn(b, 1, t, S).half().transpose(-1, -2).contiguous().transpose(-1, -2)          # columns first, one per sequence
 	assert torch.equal(aligned_mask(own), own)
 	assert aligned_mask(None) is None and aligned_mask(mask > 0) .dtype == torch.bool
+
+
+def test_projections_that_store_many_cache_rows_do_not_start_their_successor_early():
+	"""Attention reads old cache rows ahead of its wait for the kernel in front.  By the source: the prompt projection waits before
+	its first copy and never triggers, the decode projections trigger for one token per sequence only, dec_kernel not before its own wait."""
+	from gptq_triton_b200.build import CSRC
+	prompt = (CSRC / 'qmm_tc_kernel.inl').read_text()
+	assert 'pdl_trigger();' not in prompt and prompt.count('pdl_wait();') == 1
+	assert prompt.index('pdl_wait();') < min(prompt.index(call) for call in ('tma_load_2d(', 'tc_bulk_load('))
+	for name, count in (('qmm_dec.cu', 1), ('qmm_skinny.cuh', 2)):
+		text = (CSRC / name).read_text()
+		lines = [line for line in text.splitlines() if 'pdl_trigger();' in line]
+		assert len(lines) == count and sum('tokens_per_batch == 1' in line for line in lines) == 1          # the other one: gather_x_kernel
+		if name == 'qmm_dec.cu':
+			assert text.index('pdl_wait();') < text.index('pdl_trigger();')
