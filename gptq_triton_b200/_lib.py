@@ -204,10 +204,15 @@ def kernel_status(device=None) -> int:
 
 
 def clear_kernel_status():
-	"""Resets the status words (after the cause of a non-zero status has been dealt with)."""
-	for ws in _workspaces.values():
-		ws[16384 - 4:16384].zero_()
-	for ref in _status_buffers:
-		buf = ref()
-		if buf is not None:
-			buf[:16384].zero_()          # also the barrier counters, which a failed run leaves behind
+	"""Resets the status words (after the cause of a non-zero status has been dealt with) and, with them, the whole control area of every
+	scratch buffer: arrival counters, hand-over flags and barriers, which a launch that gave up leaves behind and which the next one would
+	take for its own.  Buffers that only captured graphs still use are among them.  Waits for the devices, since the buffers belong to
+	several streams."""
+	buffers = [*_workspaces.values(), *_retired, *(buf for buf in (ref() for ref in _status_buffers) if buf is not None)]
+	devices = {buf.device for buf in buffers if buf.is_cuda}
+	for device in devices:
+		torch.cuda.synchronize(device)
+	for buf in buffers:
+		buf[:16384].zero_()
+	for device in devices:
+		torch.cuda.synchronize(device)

@@ -52,7 +52,9 @@ int gptq_last_cuda_error(void);
  * problem of this size (split-K partial sums, per-tile arrival counters, and for act-order
  * decode calls the gathered copy of x).  The
  * caller allocates it once per stream, ZEROES it once, and hands it to every call;
- * the kernels leave the counter area zeroed again.  Two calls that overlap on the
+ * the kernels leave the counter area (the first 16 KiB, status word in its last 4 bytes) zeroed again, except
+ * after a non-zero status: a launch that gave up leaves counters and hand-over flags behind, so wait for the
+ * stream and zero the first 16 KiB before the next call.  Two calls that overlap on the
  * GPU must not share one workspace.  Replaces the `torch.empty` + 1-D launch grid
  * set-up of the reference wrapper (quant_linear.py:259-263).
  */

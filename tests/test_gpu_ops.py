@@ -743,3 +743,26 @@ def test_attention_with_an_odd_number_of_keys(G, b):
 	ref, _, want = attn(x, attention_mask=mask, past_key_value=kv, use_cache=True, output_attentions=True)
 	assert O.max_rel_err(y, ref.float().cpu()) <= 4 * TOL          # the other path rounds scores and weights to fp16
 	assert all(torch.equal(a, c) for a, c in zip(present, want))
+
+
+def test_decode_after_a_launch_that_gave_up(G):
+	"""Hand-over flags that an aborted launch left set (here written by the test, with a status) do not reach the launches after
+	clear_kernel_status()."""
+	from gptq_triton_b200 import _lib
+	M, K, N, gs = 16, 4096, 512, 128
+	t = synth(K, N, gs, 1)
+	args = (t['qweight'].cuda(), t['scales'].cuda(), t['qzeros'].cuda())
+	try:
+		_lib.lib().gptq_debug_dec_min_rows(1)
+		for seed in range(4):
+			x = acts((M, K), seed=seed)
+			ws = _lib.workspace(torch.device('cuda', torch.cuda.current_device()), M, K, N)
+			ws[:1024].view(torch.int32).fill_(1)
+			ws[16384 - 4:16384].view(torch.int32).fill_(6)
+			assert _lib.kernel_status() == 6
+			_lib.clear_kernel_status()
+			y = G.qmatmul(gs, x.cuda(), *args)
+			assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs)) <= TOL
+			assert _lib.kernel_status() == 0
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
