@@ -325,9 +325,13 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 	if (gather_off == (size_t)-1 && !narrow && p.M <= 8 && p.splitk > 1 &&
 		(int)(grid.x * grid.y) <= sm_count() * (kw == 2 ? 2 : 1) && ws_bytes >= words_offset(need) + words_bytes(p.M, need))
 		p.ws_words = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(workspace) + words_offset(need));
+	// the tensor-memory kernel, where it is the faster one and the workspace has room for its scratch (and the gathered x behind that)
+	const size_t dec_need = p.perm ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
+	const bool dec = gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow &&
+					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
 	if (p.perm) {
-		// act-order: x[:, perm] once, into the workspace behind the partial sums (or at the offset the caller planned)
-		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(std::max(words_offset(need) + words_bytes(p.M, need), dec_ws_bytes(p.M)));
+		// act-order: x[:, perm] once, into the workspace behind the chosen kernel's scratch (or at the offset the caller planned)
+		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(dec ? dec_ws_bytes(p.M) : words_offset(need) + words_bytes(p.M, need));
 		if (ws_bytes < off + gather_bytes(p.M, p.K)) return GPTQ_ERR_WORKSPACE;
 		__half *xp = reinterpret_cast<__half *>(reinterpret_cast<unsigned char *>(workspace) + off);
 		const dim3 gg((unsigned)((p.K / 8 + 255) / 256), (unsigned)p.M, 1);
@@ -336,8 +340,7 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 		p.ldx = p.K;
 		p.perm = nullptr;
 	}
-	if (gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow && p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) &&
-		ws_bytes >= dec_ws_bytes(p.M)) {
+	if (dec) {
 		DecArgs a = {};
 		a.x = p.x; a.ldx = p.ldx;
 		a.qw0 = qw0; a.qw1 = qw1; a.qz0 = p.qz0; a.qz1 = p.qz1; a.sc0 = p.sc0; a.sc1 = p.sc1;

@@ -766,3 +766,34 @@ def test_decode_after_a_launch_that_gave_up(G):
 			assert _lib.kernel_status() == 0
 	finally:
 		_lib.lib().gptq_debug_dec_min_rows(0)
+
+
+@pytest.mark.parametrize('M', [1, 8, 9, 16])
+@pytest.mark.parametrize('act', [False, True])
+def test_decode_workspace_without_room_for_the_tensor_memory_kernel(G, M, act):
+	"""A workspace that holds the scratch of the other decode kernel (and the gathered x of an act-order layer) and no more is enough: the
+	call runs there, with the same results, and nothing behind the workspace is touched."""
+	from gptq_triton_b200 import _lib
+	from gptq_triton_b200.quant_linear import _act_order_perm, act_order_rows
+	K, N, gs = 512, 128, 128
+	t = synth(K, N, gs, seed=M, act_order=act)
+	x = acts((M, K), seed=M + 1)
+	qw, perm = t['qweight'].cuda(), None
+	if act:
+		perm = _act_order_perm(t['g_idx'].cuda(), gs)
+		qw = act_order_rows(qw, perm)
+	up = lambda n: (n + 255) // 256 * 256
+	base = 16384 + 16 * 2 * M * 128 * 4          # counters; 16 splits x two weight streams x rows x 128 columns of fp32
+	size = up(base) + (2 * (base - 16384) if M <= 8 else 0)
+	size = up(size) + M * K * 2
+	assert size < _lib.lib().gptq_workspace_bytes(M, K, N)
+	ws = torch.zeros(size + 4096, dtype=torch.uint8, device='cuda')
+	ws[size:] = 0x5A
+	xd, sc, qz, y = x.cuda(), t['scales'].cuda(), t['qzeros'].cuda(), torch.empty((M, N), dtype=torch.float16, device='cuda')
+	P = _lib.ptr
+	for _ in range(2):
+		y.fill_(float('nan'))
+		rc = _lib.lib().gptq_qmatmul(P(xd), P(qw), P(qz), P(sc), None, P(perm), None, None, 0, P(y), M, K, N, gs, K, N, P(ws), size, _lib.stream_ptr(xd.device))
+		assert rc == 0, rc
+		assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, g_idx=t['g_idx'] if act else None)) <= TOL
+	assert not ws[:16384].any() and bool((ws[size:] == 0x5A).all())
