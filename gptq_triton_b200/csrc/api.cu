@@ -237,11 +237,25 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 	grid = dim3(tiles, p.splitk, 1);
 }
 
-// Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one.  Its time hardly depends on the rows, its start and end cost
-// about 4 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor memory / this
-// kernel: 4096 -> 4096 (8 MB) M = 4 8.5 / 7.4, M = 8 8.5 / 10.1; 11008 -> 4096 (23 MB) M = 4 11.7 / 11.2, M = 8 11.9 / 13.9;
-// 22016 -> 8192 (90 MB) M = 1 25.9 / 23.8, M = 4 26.1 / 28.8, M = 16 28.2 / 55.3; gate/up 8192 -> 2 x 22016 (180 MB) M = 1 48.5 / 48.0, M = 16 61 / 110.
-static int dec_min_rows(int K, int N, int nstream) {
+// Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one; 17: never.  Its time hardly depends on the rows, its start and
+// end cost about 4 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor
+// memory / this kernel, over 180 shapes of 0.03 to 101 MB (dependent launches, weights from HBM):
+//   4096 -> 4096 (8 MB)         M = 4   8.2 / 7.2    M = 7   8.3 / 9.6    M = 9   8.7 / 10.6   M = 16   9.8 / 11.5
+//   11008 -> 4096 (23 MB)       M = 4  11.7 / 11.3   M = 6  11.8 / 12.9   M = 9  12.4 / 17.2   M = 16  13.4 / 18.3
+//   22016 -> 8192 (90 MB)       M = 4  25.9 / 28.9   M = 6  26.0 / 54.2   M = 9  27.2 / 47.9   M = 16  28.1 / 55.3
+//   gate/up 1024 -> 2 x 1024    M = 4   6.2 / 6.8    M = 7   6.2 / 9.5    M = 9   7.0 / 11.6   M = 16   7.2 / 12.8
+//   gate/up 8192 -> 2 x 11008   M = 4  28.4 / 29.9   M = 7  28.9 / 36.5   M = 9  32.0 / 54.5   M = 16  34.5 / 66.5
+// A narrow layer with a deep K is the exception: every tile of 128 columns is spread over many CTAs, and the last one adds their sums.
+//   4096 -> 2048 (16 tiles)     M = 7   7.9 / 6.8    M = 9   8.3 / 8.3    M = 16  9.6 / 8.8
+//   8192 -> 1024 (8 tiles)      M = 7   9.9 / 8.5    M = 9  10.1 / 9.2    M = 16 12.3 / 9.7
+//   8192 -> 3072 (24 tiles)     M = 8   9.7 / 9.0    M = 9  10.2 / 11.2   M = 16 11.2 / 11.9
+//   QKV 4096 -> 1536 (12)       M = 7  10.3 / 7.8    M = 9  11.0 / 10.7   M = 16 11.2 / 11.4
+//   QKV 4096 -> 3072 (24)       M = 7   9.8 / 9.2    M = 9  10.4 / 11.5   M = 16 10.6 / 12.5
+//   QKV 4096 -> 3840 (30)       M = 7  10.2 / 10.9
+//   2048 -> 2048 (16)           M = 7   5.4 / 6.3;   QKV 1536 -> 3072 (24)   M = 7   8.2 / 7.5
+static int dec_min_rows(int K, int N, int nstream, bool rope) {
+	const int tiles = N / 128;
+	if (nstream == 1 && tiles < 30 && (rope ? K >= 1536 : K > 2048)) return tiles <= 16 ? 17 : 9;
 	const double mb = (double)K * N * nstream / 2e6;
 	return mb >= 64 ? 4 : mb >= 20 ? 6 : 7;
 }
@@ -328,7 +342,7 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 	// the tensor-memory kernel, where it is the faster one and the workspace has room for its scratch (and the gathered x behind that)
 	const size_t dec_need = p.perm ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
 	const bool dec = gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow &&
-					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
+					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM, EPI == EPI_ROPE)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
 	if (p.perm) {
 		// act-order: x[:, perm] once, into the workspace behind the chosen kernel's scratch (or at the offset the caller planned)
 		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(dec ? dec_ws_bytes(p.M) : words_offset(need) + words_bytes(p.M, need));

@@ -797,3 +797,28 @@ def test_decode_workspace_without_room_for_the_tensor_memory_kernel(G, M, act):
 		assert rc == 0, rc
 		assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, g_idx=t['g_idx'] if act else None)) <= TOL
 	assert not ws[:16384].any() and bool((ws[size:] == 0x5A).all())
+
+
+@pytest.mark.parametrize('kind,K,N,M,tensor_memory', [
+	('plain', 4096, 2048, 8, False), ('plain', 4096, 2048, 16, False), ('plain', 8192, 1024, 12, False), ('plain', 4096, 3072, 8, False),
+	('plain', 4096, 3072, 9, True), ('plain', 2048, 2048, 7, True), ('plain', 2176, 2048, 16, False), ('plain', 4096, 3840, 7, True),
+	('plain', 4096, 4096, 6, False), ('plain', 11008, 4096, 5, False), ('plain', 11008, 4096, 6, True), ('rope', 1408, 3072, 7, True),
+	('rope', 1536, 3072, 8, False), ('rope', 1536, 3072, 9, True), ('rope', 4096, 1536, 16, False), ('rope', 4096, 3840, 7, True)])
+def test_which_decode_kernel_runs(G, kind, K, N, M, tensor_memory):
+	"""Both sides of the rule that chooses the decode kernel: the call gives the bits of the kernel that it should run on.  (The two add in
+	different orders, so their results differ somewhere.)"""
+	from gptq_triton_b200 import _lib
+	t = synth(K, N, 128, 1)
+	args = (t['qweight'].cuda(), t['scales'].cuda(), t['qzeros'].cuda())
+	x = acts((1, M, K), seed=M).cuda()
+	cos, sin = (v.cuda() for v in O.rope_tables(128, 64))
+	pos = torch.arange(M, device='cuda').unsqueeze(0)
+	outs = []
+	try:
+		for rows in (0, 1, 17):          # chosen by size; tensor memory; the other one
+			_lib.lib().gptq_debug_dec_min_rows(rows)
+			outs.append(torch.cat([v.flatten() for v in G.qkv_rope(128, x, *args, cos, sin, pos, N // 384, 128)]) if kind == 'rope' else G.qmatmul(128, x, *args))
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	assert not torch.equal(outs[1], outs[2])
+	assert torch.equal(outs[0], outs[1] if tensor_memory else outs[2])
