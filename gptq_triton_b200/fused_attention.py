@@ -105,14 +105,15 @@ def qkv_rope(groupsize: int, a: torch.Tensor, qweight, scales, qzeros, cos, sin,
 
 
 def aligned_mask(mask: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-	"""The same additive mask [b, 1, t, S] with rows that start on 16 bytes.  The softmax kernel takes a much slower path for rows that do
-	not: t = 701, S = 765, 32 heads 191 us as given, 51 us with padded rows (the copy takes 3 us), t = S = 300 42 and 27 us; below about
-	180 x 180 both take 20 us and the copy does not pay."""
+	"""The same additive mask [b, 1, t, S] with rows that start on 16 bytes.  For more than 128 queries the softmax kernel takes a much slower
+	path for rows that do not (us, mask as given / copied into padded rows, the copy included; 16 to 64 heads, 1 to 8 sequences): t = 160, S = 401
+	64 / 30, t = 300, S = 301 89 / 29, t = 701, S = 765 188 / 51; at t = 181, S = 183 a call that the host bounds takes 34 / 36.  Up to 128 queries it
+	does not, and the copy is a loss: t = 33, S = 1001 30 / 37, t = 128, S = 2047 61 / 70, per call of a layer 18 / 33 at t = 64, S = 401."""
 	if mask is None or not mask.is_floating_point():
 		return mask
 	t, S = mask.shape[-2:]
 	align = 16 // mask.element_size()
-	if t * S < 1 << 15 or (mask.stride(-1) == 1 and mask.stride(-2) % align == 0):
+	if t <= 128 or t * S < 1 << 15 or (mask.stride(-1) == 1 and mask.stride(-2) % align == 0):
 		return mask
 	one = mask[:1] if mask.stride(0) == 0 else mask          # a mask shared by the batch is copied once
 	return nn.functional.pad(one, (0, -S % align))[..., :S].expand(mask.shape)

@@ -149,15 +149,15 @@ def test_bench_reference_arm_prints_one_json_line():
 	assert line['e2e'] == {'value': line['value'], 'unit': 'tokens/s', 'h2d_bytes_per_step': 0, 'd2h_bytes_per_step': 0}
 
 
-@pytest.mark.parametrize('b,t,S', [(1, 200, 265), (3, 200, 265), (1, 256, 264), (2, 3, 5)])
+@pytest.mark.parametrize('b,t,S', [(1, 200, 265), (3, 200, 265), (1, 256, 264), (2, 3, 5), (1, 128, 401), (2, 33, 2001), (1, 129, 401)])
 def test_aligned_mask_has_the_same_values(b, t, S):
-	"""Rows of a large additive mask start on 16 bytes afterwards; values, shape and the sharing over the batch stay, small masks and
-	masks of truth values are passed on."""
+	"""Rows of a large additive mask start on 16 bytes afterwards; values, shape and the sharing over the batch stay; small masks, masks of
+	up to 128 queries (for which the copy does not pay) and masks of truth values are passed on."""
 	from gptq_triton_b200.fused_attention import aligned_mask
 	mask = torch.randn(1, 1, t, S).half().expand(b, 1, t, S)
 	out = aligned_mask(mask)
 	assert out.shape == mask.shape and torch.equal(out, mask)
-	if t * S < 1 << 15:
+	if t <= 128 or t * S < 1 << 15:
 		assert out is mask
 	else:
 		assert out.stride(-1) == 1 and out.stride(-2) % 8 == 0 and (b == 1 or out.stride(0) == 0)
