@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 			if (!tc_wait(bar, ph, s_abort)) { fail(); break; }
 			tc_fence_after();
 			if (one) {
-				// (where K ends on an odd block, the second block of the last stage is zero in X)
+				// (where K ends on an odd block, the second block of the last stage is zero in X and in the weights)
 #pragma unroll
 				for (int k = 0; k < KP * TC_BK / 16; ++k)
 					umma_f16_ts(tmem, at + 8 * k, xd + (uint64_t)((k >> 2) * (x_block >> 4) + 2 * (k & 3)), idesc, k == 0 ? acc : 1u);
@@ -193,6 +193,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_kernel(const __grid_constant
 				for (int r = 0; r < 8; ++r) w[r] = tc_lds32(st + w_off + (8 * h + r) * W_ROW);
 				if (h == 0 || sets == 2) {
 					sc = tc_lds16(st + W_SC + h * 256 + wt * 2) * 0x00010001u;
+					// behind an odd number of K-blocks: exact zeros.  (0 - zero) * scale may be infinite in fp16, times the zeros of X a NaN
+					if (KP == 2 && h == 1 && 2 * i + 1 >= nkb) sc = 0u;
 					const uint32_t zz = ((tc_lds32(st + W_QZ + h * 64 + (wt >> 3) * 4) >> zsh) & 0xFu) + 1u;
 					ze = (0x6400u + zz) * 0x00010001u;            // half2(1024 + zero)
 					zo = (0xD400u + (zz << 4)) * 0x00010001u;     // half2(-(64 + zero))

@@ -822,3 +822,24 @@ def test_which_decode_kernel_runs(G, kind, K, N, M, tensor_memory):
 		_lib.lib().gptq_debug_dec_min_rows(0)
 	assert not torch.equal(outs[1], outs[2])
 	assert torch.equal(outs[0], outs[1] if tensor_memory else outs[2])
+
+
+@pytest.mark.parametrize('M', [17, 40, 144, 145])
+@pytest.mark.parametrize('K,gs', [(192, 64), (448, 64), (192, 192)])
+def test_prefill_of_large_scales_behind_an_odd_number_of_k_blocks(G, M, K, gs):
+	"""Finite weights near the end of fp16's range, with zero points that only the codes in use keep finite: what pads an odd number of
+	K-blocks of 64 to whole stages (code 0, zero point 16, scale 5000) must not reach the sums."""
+	from gptq_triton_b200 import _lib
+	H, D = 2, 128
+	rng = np.random.default_rng(K + M)
+	codes = rng.integers(3, 16, size=(K // 8, 8, 3 * H * D)).astype(np.uint32)          # (3 - 16) * 5000 = -65000
+	qweight = torch.from_numpy((codes << (4 * np.arange(8, dtype=np.uint32))[None, :, None]).sum(1, dtype=np.uint32).view(np.int32))
+	qzeros = torch.full((K // gs, 3 * H * D // 8), -1, dtype=torch.int32)               # stored 15: zero point 16
+	scales = torch.full((K // gs, 3 * H * D), 5000.0).half()
+	x = (1e-4 * acts((1, M, K), seed=M).float()).half()
+	pos = torch.arange(M).unsqueeze(0)
+	cos, sin = O.rope_tables(D, 256)
+	got = G.qkv_rope(gs, x.cuda(), qweight.cuda(), scales.cuda(), qzeros.cuda(), cos.cuda(), sin.cuda(), pos.cuda(), H, D)
+	for y, ref in zip(got, O.qkv_rope_r32(x, qweight, qzeros, scales, gs, cos, sin, pos, H, D)):
+		assert bool(torch.isfinite(y).all()) and O.max_rel_err(y.transpose(1, 2), ref) <= TOL
+	assert _lib.kernel_status() == 0
