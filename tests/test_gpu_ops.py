@@ -608,12 +608,14 @@ def test_decode_narrow_geometry(G, M, K, gs):
 	d = {k: dev(v) for k, v in t.items() if isinstance(v, torch.Tensor)}
 	ss = torch.zeros((M, N // 32), dtype=torch.float32, device='cuda')
 	ss2 = torch.zeros_like(ss)
-	y2 = G.qmatmul(gs, x.cuda(), d['qweight'], d['scales'], d['qzeros'], bias=d['bias'], residual=res.cuda(), sumsq_out=ss2)      # tiled split-K form
 	try:
+		_lib.lib().gptq_debug_dec_min_rows(17)          # not the tensor-memory kernel
+		y2 = G.qmatmul(gs, x.cuda(), d['qweight'], d['scales'], d['qzeros'], bias=d['bias'], residual=res.cuda(), sumsq_out=ss2)      # tiled split-K form
 		_lib.lib().gptq_debug_allow_narrow(1)
 		y = G.qmatmul(gs, x.cuda(), d['qweight'], d['scales'], d['qzeros'], bias=d['bias'], residual=res.cuda(), sumsq_out=ss)
 	finally:
 		_lib.lib().gptq_debug_allow_narrow(0)
+		_lib.lib().gptq_debug_dec_min_rows(0)
 	r32 = O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, bias=t['bias'], residual=res)
 	assert O.max_rel_err(y, r32) <= 6e-4 and O.max_rel_err(y2, r32) <= 6e-4
 	assert torch.allclose(ss, y.float().pow(2).view(M, N // 32, 32).sum(-1), rtol=1e-5, atol=1e-6)
@@ -643,10 +645,21 @@ def test_row_parallel_shards_of_an_act_order_layer_on_the_gpu(G):
 @pytest.mark.parametrize('sk', [2, 4])
 @pytest.mark.parametrize('cfg', [1, 2, 3, 4])
 def test_prefill_split_k(G, cfg, sk):
-	"""Split-K of the tensor-core kernel (plain epilogue): every tile configuration with 2 and 4 splits, uneven last
-	split (K = 1216 = 19 blocks of 64), bias and residual applied by the finishing kernel."""
+	"""K = 1216 = 19 blocks of 64: no multiple of 128, so a single projection runs on the general kernel whatever the hooks say."""
+	check_split_k(G, cfg, sk, 1216)
+
+
+@pytest.mark.parametrize('sk', [2, 3, 4])
+@pytest.mark.parametrize('cfg', [1, 2, 3, 4])
+def test_prefill_split_k_on_the_tensor_cores(G, cfg, sk):
+	"""Split K of the tensor-core kernel (plain epilogue): every cap on the rows of a tile with 2 to 4 splits, an uneven last split
+	(K = 1408 = 22 blocks of 64 in ranges of 12, 8 or 6), bias and residual added after the sums of the cluster."""
+	check_split_k(G, cfg, sk, 1408)
+
+
+def check_split_k(G, cfg, sk, K):
 	from gptq_triton_b200 import _lib
-	M, K, N, gs = 300, 1216, 512, 64
+	M, N, gs = 300, 512, 64
 	t = synth(K, N, gs, seed=cfg * 10 + sk, bias=True)
 	x, res = acts((M, K), seed=3), acts((M, N), seed=4)
 	ref = O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs, bias=t['bias'], residual=res)
@@ -663,10 +676,12 @@ def test_prefill_split_k(G, cfg, sk):
 
 
 @pytest.mark.parametrize('sk', [1, 3, 8])
-@pytest.mark.parametrize('M,K,gs', [(17, 1984, 64), (33, 1024, -1), (144, 1920, 128), (145, 1984, 64), (256, 1024, 512), (257, 1920, 192)])
+@pytest.mark.parametrize('M,K,gs', [(17, 1984, 64), (33, 1024, -1), (144, 1920, 128), (145, 1984, 64), (256, 1024, 512), (257, 1920, 192),
+									(17, 1920, 64), (145, 1920, 64), (257, 1920, 384)])
 def test_prefill_edges_of_row_tiles_and_splits(G, M, K, gs, sk):
 	"""Rows just below and above a tile of the tensor-core kernel (stages of two K-blocks up to 144 rows, one above; 256 rows per tile),
-	odd numbers of K-blocks, groups that end inside a stage, and clusters of 1, 3 and 8 CTAs, with every epilogue."""
+	groups that end inside a stage, and clusters of 1, 3 and 8 CTAs, with every epilogue.  Odd numbers of K-blocks (K = 1984) and groups of 192
+	reach it with the rotary epilogue; the other two run on the general kernel there."""
 	from gptq_triton_b200 import _lib
 	H, D, N = 2, 128, 256
 	t, g, u, w = synth(K, N, gs, 1, bias=True), synth(K, N, gs, 2), synth(K, N, gs, 3), synth(K, 3 * H * D, gs, 4)
@@ -843,3 +858,65 @@ def test_prefill_of_large_scales_behind_an_odd_number_of_k_blocks(G, M, K, gs):
 	for y, ref in zip(got, O.qkv_rope_r32(x, qweight, qzeros, scales, gs, cos, sin, pos, H, D)):
 		assert bool(torch.isfinite(y).all()) and O.max_rel_err(y.transpose(1, 2), ref) <= TOL
 	assert _lib.kernel_status() == 0
+
+
+@pytest.fixture
+def mma_sync_kernel():
+	"""Decode calls of any number of rows on the mma.sync kernel, which the tensor-memory kernel otherwise replaces for several rows."""
+	from gptq_triton_b200 import _lib
+	_lib.lib().gptq_debug_dec_min_rows(17)
+	yield
+	_lib.lib().gptq_debug_dec_min_rows(0)
+
+
+@pytest.mark.parametrize('K,N,gs', SHAPES)
+@pytest.mark.parametrize('M', [8, 9, 16])
+def test_mma_sync_kernel_plain(G, mma_sync_kernel, M, K, N, gs):
+	test_qmatmul_decode(G, M, K, N, gs)
+
+
+@pytest.mark.parametrize('M', [7, 16])
+@pytest.mark.parametrize('K,N,gs', [(256, 256, 128), (4096, 1376, 128), (512, 512, -1)])
+def test_mma_sync_kernel_gateup(G, mma_sync_kernel, M, K, N, gs):
+	test_gateup_silu_decode(G, M, K, N, gs)
+
+
+@pytest.mark.parametrize('b,t', [(4, 2), (4, 4), (1, 16)])
+@pytest.mark.parametrize('ao', [False, True])
+def test_mma_sync_kernel_qkv_rope(G, mma_sync_kernel, b, t, ao):
+	test_qkv_rope_decode(G, b, t, ao)
+
+
+@pytest.mark.parametrize('M', [8, 16])
+def test_mma_sync_kernel_folded_rmsnorm(G, mma_sync_kernel, M):
+	test_rmsnorm_folded_into_decode_kernels(G, M)
+
+
+@pytest.mark.parametrize('b,t', [(1, 1), (8, 1), (2, 8), (2, 20), (1, 150)])
+def test_rotary_outputs_that_do_not_start_on_8_bytes(G, b, t):
+	"""Q, K and V with rows, heads and sequences an even but no multiple of four halfs apart (through the C ABI): the same values as with packed
+	outputs, and what lies between the rows stays."""
+	from gptq_triton_b200 import _lib
+	H, D, K, gs, M = 2, 128, 512, 128, b * t
+	w = synth(K, 3 * H * D, gs, seed=3)
+	qw, sc, qz = w['qweight'].cuda(), w['scales'].cuda(), w['qzeros'].cuda()
+	x = acts((b, t, K), seed=4).cuda()
+	cos, sin = (v.cuda() for v in O.rope_tables(D, 256))
+	pos = torch.arange(t, dtype=torch.int32, device='cuda').repeat(b)
+	P, st = _lib.ptr, _lib.stream_ptr(x.device)
+	ws = _lib.workspace(x.device, M, K, 3 * H * D)
+	try:
+		_lib.lib().gptq_debug_dec_min_rows(7)          # 8 and 16 rows: the tensor-memory kernel
+		want = G.qkv_rope(gs, x, qw, sc, qz, cos, sin, pos.view(b, t), H, D)
+		head, row, q_row = D + 2, H * (D + 2), H * D + 2
+		q = torch.full((M, q_row), 7.0, dtype=torch.float16, device='cuda')
+		k, v = (torch.full((b, t, H, head), 7.0, dtype=torch.float16, device='cuda') for _ in range(2))
+		rc = _lib.lib().gptq_qkv_rope(P(x), P(qw), P(qz), P(sc), None, None, P(cos), P(sin), P(pos), cos.shape[0], P(q), q_row, P(k), P(v), t, t * row, row,
+									  head, 0, M, K, H, D, gs, K, P(ws), ws.numel(), st)
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	assert rc == 0
+	assert torch.equal(q[:, :H * D].view(b, t, H, D).transpose(1, 2), want[0])
+	for got, ref in ((k, want[1]), (v, want[2])):
+		assert torch.equal(got[..., :D].transpose(1, 2), ref) and bool((got[..., D:] == 7.0).all())
+	assert bool((q[:, H * D:] == 7.0).all()) and _lib.kernel_status() == 0
