@@ -249,10 +249,10 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 //   4096 -> 2048 (16 tiles)     M = 7   7.9 / 6.8    M = 9   8.3 / 8.3    M = 16  9.6 / 8.8
 //   8192 -> 1024 (8 tiles)      M = 7   9.9 / 8.5    M = 9  10.1 / 9.2    M = 16 12.3 / 9.7
 //   8192 -> 3072 (24 tiles)     M = 8   9.7 / 9.0    M = 9  10.2 / 11.2   M = 16 11.2 / 11.9
-//   QKV 4096 -> 1536 (12)       M = 7  10.3 / 7.8    M = 9  11.0 / 10.7   M = 16 11.2 / 11.4
-//   QKV 4096 -> 3072 (24)       M = 7   9.8 / 9.2    M = 9  10.4 / 11.5   M = 16 10.6 / 12.5
-//   QKV 4096 -> 3840 (30)       M = 7  10.2 / 10.9
-//   2048 -> 2048 (16)           M = 7   5.4 / 6.3;   QKV 1536 -> 3072 (24)   M = 7   8.2 / 7.5
+//   QKV 4096 -> 1536 (12)       M = 7  10.5 / 7.7    M = 9  11.2 / 10.7   M = 16 11.4 / 11.4
+//   QKV 4096 -> 3072 (24)       M = 7   9.9 / 9.4    M = 9  10.6 / 11.5   M = 16 10.8 / 12.3
+//   QKV 4096 -> 3840 (30)       M = 7  10.4 / 10.9   (QKV: one token per sequence)
+//   2048 -> 2048 (16)           M = 7   5.4 / 6.3;   QKV 1536 -> 3072 (24)   M = 7   8.4 / 7.6
 static int dec_min_rows(int K, int N, int nstream, bool rope) {
 	const int tiles = N / 128;
 	if (nstream == 1 && tiles < 30 && (rope ? K >= 1536 : K > 2048)) return tiles <= 16 ? 17 : 9;

@@ -5,8 +5,8 @@
 // holds the INTEGERS q - zero as fp16, which is exact; a unit of 128 K-rows lies in one group, so its fp32 sums leave tensor memory, are
 // multiplied with the group's scale in fp32 and added in registers.  No weight is rounded.
 //
-// Split of the work: one CTA per SM; the units of all tiles (128 columns, or 64 gate + 64 up) x K / 128 are one list that is cut into equal
-// ranges, so that every SM streams the same number of bytes whatever the shape.  A CTA walks its tiles from the last to the first: the tile
+// Split of the work: one CTA per SM, fewer when there are less than two units for each; the units of all tiles (128 columns, or 64 gate + 64 up)
+// x K / 128 are one list that is cut into ranges which differ by at most one unit of 128 x 128 weights.  A CTA walks its tiles from the last to the first: the tile
 // whose end lies in the next CTA's range comes first and its partial sums are handed over early, the tile whose beginning lies in the
 // ranges of earlier CTAs comes last and is finished there (partial sums added in order of K: deterministic).  A CTA only ever waits for
 // CTAs with lower indices.
@@ -20,8 +20,9 @@
 //
 // What bounds it: the instructions around a unit (0.21 - 0.25 us per unit and CTA, 3.2 - 3.7 TB/s of weights at 90 MB and more) and about
 // 8 us from launch to exit (prologue, first copies, hand-over).  Measured against the mma.sync kernel (qmm_skinny.cuh), us, 16 rows:
-//   4096 -> 4096 10.1 (11.8)   4096 -> 12288 13.9 (18.1)   11008 -> 4096 13.4 (18.3)   8192 -> 24576 31.7 (57.3)   22016 -> 8192 28.2 (55.3)
-//   gate/up 4096 -> 2 x 11008 21.5 (34.8)   8192 -> 2 x 22016 61 (110)
+//   4096 -> 4096 10.3 (11.7)   4096 -> 12288 14.4 (18.0)   11008 -> 4096 13.5 (18.3)   8192 -> 24576 32.0 (57.1)   22016 -> 8192 28.6 (55.6)
+//   gate/up 4096 -> 2 x 11008 21.8 (34.8)   8192 -> 2 x 22016 61 (110)
+// On narrow layers with a deep K, where a tile is spread over many CTAs, it is the slower one; dec_min_rows() in api.cu draws the line.
 // A spilled register in a loop costs an L2 round trip (shared memory takes the whole L1): with spills the last line read 154 us.
 //
 // Every wait is bounded; a wait that runs out sets a status word and the kernel unwinds.

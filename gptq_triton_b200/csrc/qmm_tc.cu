@@ -23,10 +23,10 @@
 // What bounds it: up to about 130 rows the issue slots of the dequantisation (17 instructions per 8 weights), above the MMAs and, from
 // about 1000 rows, the power limit (1250 - 1430 TFLOP/s; cuBLAS bf16: 1670 in a burst, 1410 sustained).  Measured, in brackets the
 // kernel with both operands in shared memory that this one replaced (us; 128-row tiles, split K through global memory):
-//   M = 17    4096 -> 12288  12.3 (26.3)   22016 -> 8192  30.4 (56.2)   gate/up 8192 -> 2 x 22016   69 (190)
-//   M = 203   4096 -> 12288  22.1 (46.8)   22016 -> 8192  58.5 (84.2)   gate/up 8192 -> 2 x 22016  126 (247)
-//   M = 512   4096 -> 4096   17.0 (36.0)   11008 -> 4096  36.3 (55.8)   gate/up 4096 -> 2 x 11008   86 (132)
-//   M = 2048  4096 -> 4096   53.2 (58.0)   11008 -> 4096   134 (145)    gate/up 4096 -> 2 x 11008  296 (332)
+//   M = 17    4096 -> 12288  13.8 (26.3)   22016 -> 8192  31.4 (56.2)   gate/up 8192 -> 2 x 22016   73 (190)
+//   M = 203   4096 -> 12288  22.8 (46.8)   22016 -> 8192  60.6 (84.2)   gate/up 8192 -> 2 x 22016  130 (247)
+//   M = 512   4096 -> 4096   17.9 (36.0)   11008 -> 4096  38.0 (55.8)   gate/up 4096 -> 2 x 11008   88 (132)
+//   M = 2048  4096 -> 4096   55.8 (58.0)   11008 -> 4096   139 (145)    gate/up 4096 -> 2 x 11008  302 (332)
 //
 // It keeps its place in the stream in both directions: it stores many cache rows and may be the first reader of new weights, so it reads nothing
 // ahead of its dependency wait and never triggers its successor (see pdl_trigger in common.cuh).  As a dependent launch it still has its
