@@ -238,26 +238,27 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 }
 
 // Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one; 17: never.  Its time hardly depends on the rows, its start and
-// end cost about 4 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor
-// memory / this kernel, over 180 shapes of 0.03 to 101 MB (dependent launches, weights from HBM):
-//   4096 -> 4096 (8 MB)         M = 4   8.2 / 7.2    M = 7   8.3 / 9.6    M = 9   8.7 / 10.6   M = 16   9.8 / 11.5
-//   11008 -> 4096 (23 MB)       M = 4  11.7 / 11.3   M = 6  11.8 / 12.9   M = 9  12.4 / 17.2   M = 16  13.4 / 18.3
-//   22016 -> 8192 (90 MB)       M = 4  25.9 / 28.9   M = 6  26.0 / 54.2   M = 9  27.2 / 47.9   M = 16  28.1 / 55.3
-//   gate/up 1024 -> 2 x 1024    M = 4   6.2 / 6.8    M = 7   6.2 / 9.5    M = 9   7.0 / 11.6   M = 16   7.2 / 12.8
-//   gate/up 8192 -> 2 x 11008   M = 4  28.4 / 29.9   M = 7  28.9 / 36.5   M = 9  32.0 / 54.5   M = 16  34.5 / 66.5
+// end cost about 3 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor
+// memory / this kernel (dependent launches, weights from HBM):
+//   4096 -> 4096 (8 MB)           M = 4   7.5 / 7.1    M = 7   7.6 / 9.6    M = 9   7.7 / 10.6   M = 16   8.4 / 11.5
+//   11008 -> 4096 (23 MB)         M = 4  10.9 / 11.3   M = 6  11.0 / 12.9   M = 9  11.3 / 17.2   M = 16  11.9 / 18.4
+//   4096 -> 12288 (25 MB)         M = 4  12.0 / 10.9   M = 5  12.1 / 12.3   M = 9  12.4 / 16.5   M = 16  12.9 / 17.9
+//   gate/up 4096 -> 2 x 11008     M = 3  17.5 / 17.3   M = 4  17.5 / 18.4   M = 8  17.6 / 24.1   M = 16  18.0 / 35.3
+//   22016 -> 8192 (90 MB)         M = 2  25.5 / 25.3   M = 3  25.5 / 27.9   M = 7  25.7 / 40.1   M = 16  27.0 / 55.4
+//   gate/up 8192 -> 2 x 11008     M = 2  27.2 / 26.9   M = 3  27.1 / 28.6   M = 8  27.2 / 38.3   M = 16  27.9 / 66.3
+//   8192 -> 24576 (101 MB)        M = 2  28.1 / 29.4   M = 4  28.1 / 33.8   M = 8  28.1 / 41.2   M = 16  29.4 / 57.3
+//   the same with the folded norm (a kernel of its own ahead of this one): gate/up 8192 -> 2 x 22016   M = 1  50.2 / 49.8   M = 2  51.4 / 54.2
+//   M = 16  53.7 / 119;   gate/up 4096 -> 2 x 11008   M = 3  18.4 / 18.2   M = 4  18.7 / 19.5   M = 16  19.7 / 38.0
 // A narrow layer with a deep K is the exception: every tile of 128 columns is spread over many CTAs, and the last one adds their sums.
-//   4096 -> 2048 (16 tiles)     M = 7   7.9 / 6.8    M = 9   8.3 / 8.3    M = 16  9.6 / 8.8
-//   8192 -> 1024 (8 tiles)      M = 7   9.9 / 8.5    M = 9  10.1 / 9.2    M = 16 12.3 / 9.7
-//   8192 -> 3072 (24 tiles)     M = 8   9.7 / 9.0    M = 9  10.2 / 11.2   M = 16 11.2 / 11.9
-//   QKV 4096 -> 1536 (12)       M = 7  10.5 / 7.7    M = 9  11.2 / 10.7   M = 16 11.4 / 11.4
-//   QKV 4096 -> 3072 (24)       M = 7   9.9 / 9.4    M = 9  10.6 / 11.5   M = 16 10.8 / 12.3
-//   QKV 4096 -> 3840 (30)       M = 7  10.4 / 10.9   (QKV: one token per sequence)
-//   2048 -> 2048 (16)           M = 7   5.4 / 6.3;   QKV 1536 -> 3072 (24)   M = 7   8.4 / 7.6
+//   4096 -> 2048 (16 tiles)     M = 7   7.6 / 6.8    M = 9   7.7 / 8.4    M = 16  8.5 / 8.9
+//   8192 -> 1024 (8 tiles)      M = 7   9.8 / 8.4    M = 9   9.8 / 9.2    M = 16 11.7 / 9.7
+//   8192 -> 3072 (24 tiles)     M = 8   9.2 / 9.0    M = 9   9.4 / 11.3   M = 16 10.2 / 12.0
+//   2048 -> 2048 (16)           M = 4   5.0 / 4.5    M = 7   5.0 / 6.4
 static int dec_min_rows(int K, int N, int nstream, bool rope) {
 	const int tiles = N / 128;
 	if (nstream == 1 && tiles < 30 && (rope ? K >= 1536 : K > 2048)) return tiles <= 16 ? 17 : 9;
 	const double mb = (double)K * N * nstream / 2e6;
-	return mb >= 64 ? 4 : mb >= 20 ? 6 : 7;
+	return mb >= 100 ? 2 : mb >= 64 ? 3 : mb >= 40 ? 4 : mb >= 24 ? 5 : mb >= 20 ? 6 : 7;
 }
 
 // Narrow geometry (one 32-column strip and the whole of K per CTA, no split-K): worth it when
@@ -339,8 +340,8 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 	if (gather_off == (size_t)-1 && !narrow && p.M <= 8 && p.splitk > 1 &&
 		(int)(grid.x * grid.y) <= sm_count() * (kw == 2 ? 2 : 1) && ws_bytes >= words_offset(need) + words_bytes(p.M, need))
 		p.ws_words = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(workspace) + words_offset(need));
-	// the tensor-memory kernel, where it is the faster one and the workspace has room for its scratch (and the gathered x behind that)
-	const size_t dec_need = p.perm ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
+	// the tensor-memory kernel, where it is the faster one and the workspace has room for its scratch (and the gathered or normalised x behind that)
+	const size_t dec_need = (p.perm || p.rms_w) ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
 	const bool dec = gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow &&
 					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM, EPI == EPI_ROPE)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
 	if (p.perm) {
@@ -354,13 +355,19 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 		p.ldx = p.K;
 		p.perm = nullptr;
 	}
+	if (dec && p.rms_w) {
+		__half *xn = reinterpret_cast<__half *>(reinterpret_cast<unsigned char *>(workspace) + gather_offset(dec_ws_bytes(p.M)));
+		const dim3 gn((unsigned)((p.K / 8 + 255) / 256), (unsigned)p.M, 1);
+		if (int rc = launch_ex(norm_x_kernel, gn, dim3(256, 1, 1), 0, stream, p.x, p.ldx, p.rms_w, p.ss_in, p.ss_tiles, p.rms_eps, xn, p.K)) return rc;
+		p.x = xn;
+		p.ldx = p.K;
+	}
 	if (dec) {
 		DecArgs a = {};
 		a.x = p.x; a.ldx = p.ldx;
 		a.qw0 = qw0; a.qw1 = qw1; a.qz0 = p.qz0; a.qz1 = p.qz1; a.sc0 = p.sc0; a.sc1 = p.sc1;
 		a.M = p.M; a.K = p.K; a.N = p.N; a.groupsize = p.groupsize;
 		a.bias = p.bias; a.residual = p.residual; a.ldr = p.ldr; a.y = p.y; a.ldy = p.ldy; a.ss_out = p.ss_out;
-		a.rms_w = p.rms_w; a.ss_in = p.ss_in; a.ss_tiles = p.ss_tiles; a.rms_eps = p.rms_eps;
 		a.cos_t = p.cos_t; a.sin_t = p.sin_t; a.pos = p.pos; a.q_out = p.q_out; a.k_out = p.k_out; a.v_out = p.v_out;
 		a.q_stride_m = p.q_stride_m; a.kv_sb = p.kv_sb; a.kv_st = p.kv_st; a.kv_sh = p.kv_sh; a.kv_sp = p.kv_sp;
 		a.tokens_per_batch = p.tokens_per_batch; a.hidden = p.hidden; a.max_pos = p.max_pos;

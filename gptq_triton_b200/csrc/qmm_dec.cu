@@ -2,8 +2,8 @@
 // and multiplied with all rows in one MMA.
 //
 // The product is computed transposed (a weight column is a lane of tensor memory, the rows of x are the N = 16 of the MMA).  The A operand
-// holds the INTEGERS q - zero as fp16, which is exact; a unit of 128 K-rows lies in one group, so its fp32 sums leave tensor memory, are
-// multiplied with the group's scale in fp32 and added in registers.  No weight is rounded.
+// holds the INTEGERS q - zero as fp16 (times 2^-9), which is exact; a unit of 128 K-rows lies in one group, so its fp32 sums leave tensor memory,
+// are multiplied with the group's scale in fp32 and added in registers.  No weight is rounded.
 //
 // Split of the work: one CTA per SM, fewer when there are less than two units for each; the units of all tiles (128 columns, or 64 gate + 64 up)
 // x K / 128 are one list that is cut into ranges which differ by at most one unit of 128 x 128 weights.  A CTA walks its tiles from the last to the first: the tile
@@ -11,19 +11,23 @@
 // ranges of earlier CTAs comes last and is finished there (partial sums added in order of K: deterministic).  A CTA only ever waits for
 // CTAs with lower indices.
 //
-//   warps 0, 3   packed weights (16 words x 128 columns); scales and zeros; into a ring of 18 units
-//   warp 1       MMA issuer: eight K = 16 steps per unit
-//   warp 2       owns the tensor memory (6 stages of 64 columns of weights and of 16 columns of sums)
-//   warps 4-7    rows of x, a warp per unit in turn: RMSNorm factor where asked for, k order 0 4 1 5 2 6 3 7 of each eight (as the nibbles of a word unpack in
-//                pairs), into the 128-byte-swizzled B operand
-//   warps 8-19   three groups of four; group j unpacks the units j, j + 3, ... and later scales and adds their sums
+//   warps 0, 3   packed weights (16 words x 128 columns); scales and zeros; into a ring of 15 units
+//   warp 1       MMA issuer: eight K = 16 steps per unit; owns the tensor memory (6 stages of 64 columns of weights and of 16 columns of sums)
+//   warp 2       rows of x by TMA, in the order in which they lie in memory: a pair of neighbouring nibbles is unpacked into one word
+//   warps 4-7    finish every tile but the CTA's last one (hand-over or epilogue) while the next one is unpacked
+//   warps 8-19   three groups of four; group j unpacks the units j, j + 3, ... and later scales and adds their sums; all of them finish the last tile
 //
-// What bounds it: the instructions around a unit (0.21 - 0.25 us per unit and CTA, 3.2 - 3.7 TB/s of weights at 90 MB and more) and about
-// 8 us from launch to exit (prologue, first copies, hand-over).  Measured against the mma.sync kernel (qmm_skinny.cuh), us, 16 rows:
-//   4096 -> 4096 10.3 (11.7)   4096 -> 12288 14.4 (18.0)   11008 -> 4096 13.5 (18.3)   8192 -> 24576 32.0 (57.1)   22016 -> 8192 28.6 (55.6)
-//   gate/up 4096 -> 2 x 11008 21.8 (34.8)   8192 -> 2 x 22016 61 (110)
+// What bounds it: stores to tensor memory.  A unit is 32 KB of fp16 there and takes about 0.27 us (some 64 bytes a clock; without three quarters
+// of the stores, all else equal, 0.20 us a unit, which is what the weights take from HBM), and about 6 us from launch to exit (prologue, first
+// copies, hand-over).  Measured against the mma.sync kernel (qmm_skinny.cuh), us, 16 rows:
+//   4096 -> 4096 8.4 (11.5)   4096 -> 12288 12.9 (17.9)   11008 -> 4096 11.9 (18.4)   8192 -> 24576 29.4 (57.3)   22016 -> 8192 27.0 (55.4)
+//   gate/up 4096 -> 2 x 11008 18.0 (35.3)   8192 -> 2 x 22016 50 (110)
+// What brought it there (same sizes, before: 9.7, 13.8, 13.3, 31.6, 28.4, 21.6, 61): x by TMA instead of four warps that permuted it for every
+// unit (gate/up 61 -> 54), the norm in a kernel of its own (82.6 -> 58), tiles finished beside the main loop and a hand-over without a
+// fence per thread (4 us of each launch), stores to tensor memory in four parts that overlap with the unpacking (54 -> 50).  Eight warps per
+// unit were slower (8192 -> 24576 35.4).
 // On narrow layers with a deep K, where a tile is spread over many CTAs, it is the slower one; dec_min_rows() in api.cu draws the line.
-// A spilled register in a loop costs an L2 round trip (shared memory takes the whole L1): with spills the last line read 154 us.
+// A spilled register in a loop costs an L2 round trip (shared memory takes the whole L1).
 //
 // Every wait is bounded; a wait that runs out sets a status word and the kernel unwinds.
 #include <algorithm>
@@ -37,20 +41,22 @@ namespace gptq {
 
 namespace {
 
-constexpr int DC_GROUPS = 3, DC_STAGES = 6;                  // two stages per group
-constexpr int DC_WORKERS = DC_GROUPS * 128;
-constexpr int DC_THREADS = 256 + DC_WORKERS;
+constexpr int DC_GROUPS = 3, DC_STAGES = 6;                  // three groups of four warps that unpack, two stages each
+constexpr int DC_WORKERS = DC_GROUPS * 128, DC_FINISHERS = 128;
+constexpr int DC_THREADS = 128 + DC_FINISHERS + DC_WORKERS;
 constexpr int DC_W_SC = 8192, DC_W_QZ = DC_W_SC + 256, DC_W_BYTES = DC_W_QZ + 64, DC_W_STAGE = (DC_W_BYTES + 127) / 128 * 128;
-constexpr int DC_W_RING = 18;                                // a multiple of the groups: a stage is always read by the same one
-constexpr int DC_X_STAGE = 4096;                             // 16 rows x 128 k
-constexpr int DC_RED = DC_GROUPS * 16 * 128 * 4;
-constexpr int DC_OFF_W = DC_STAGES * DC_X_STAGE, DC_OFF_RED = DC_OFF_W + DC_W_RING * DC_W_STAGE, DC_OFF_BAR = DC_OFF_RED + DC_RED;
-constexpr int DC_SMEM = DC_OFF_BAR + (2 * DC_STAGES + 2 * DC_W_RING + 1) * 8 + 16;
-constexpr int DC_D_COLS = 16, DC_TMEM_COLS = 512;
+constexpr int DC_W_RING = 15;                                // a multiple of the groups: a stage is always read by the same one
+constexpr int DC_X_BYTES = 4096;                             // 16 rows x 128 k
+constexpr int DC_RED = DC_GROUPS * 16 * 128 * 4;            // a tile's sums, one part per group; two buffers
+constexpr int DC_OFF_W = DC_STAGES * DC_X_BYTES, DC_OFF_RED = DC_OFF_W + DC_W_RING * DC_W_STAGE, DC_OFF_BAR = DC_OFF_RED + 2 * DC_RED;
+// mbarriers: weights and x of a unit are there; the unit has been multiplied; packed weights; a tile's sums; all MMAs
+constexpr int DC_FULL = DC_OFF_BAR, DC_DONE = DC_FULL + 8 * DC_STAGES, DC_FULL_W = DC_DONE + 8 * DC_STAGES, DC_EMPTY_W = DC_FULL_W + 8 * DC_W_RING;
+constexpr int DC_FULL_R = DC_EMPTY_W + 8 * DC_W_RING, DC_EMPTY_R = DC_FULL_R + 16, DC_FIN = DC_EMPTY_R + 16, DC_TMEM_ADDR = DC_FIN + 8, DC_ABORT = DC_TMEM_ADDR + 4, DC_SMEM = DC_TMEM_ADDR + 16;
+constexpr int DC_A_COLS = 64, DC_STAGE_COLS = DC_A_COLS + 16, DC_TMEM_COLS = 512;
 constexpr uint32_t DC_SPIN = 1u << 24;
 constexpr int DC_COUNTERS = 16384;                           // bytes of the workspace's counter area; its last word is the status word
 constexpr int DC_MAX_CTAS = 256;
-static_assert(DC_STAGES * (64 + DC_D_COLS) <= DC_TMEM_COLS && DC_W_RING % DC_GROUPS == 0 && DC_STAGES == 2 * DC_GROUPS, "rings");
+static_assert(DC_STAGES * DC_STAGE_COLS <= DC_TMEM_COLS && DC_W_RING % DC_GROUPS == 0 && DC_STAGES % DC_GROUPS == 0, "rings");
 static_assert(DC_SMEM + 512 <= 227 * 1024, "shared memory per CTA");
 
 struct DecParams {
@@ -62,11 +68,21 @@ struct DecParams {
 	int out8;
 };
 
-__device__ __noinline__ bool dc_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-	return __all_sync(0xffffffffu, !*abort_flag && mbar_wait_bounded(bar, parity, DC_SPIN));
+// `base`: start of the CTA's shared memory
+__device__ __forceinline__ bool dc_aborted(uint32_t base) {
+	int f;
+	asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(f) : "r"(base + DC_ABORT) : "memory");
+	return f != 0;
 }
-__device__ __forceinline__ bool dc_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-	return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || dc_wait_slow(bar, parity, abort_flag);
+__device__ __forceinline__ void dc_abort(uint32_t base, int *status, int code) {
+	asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(base + DC_ABORT), "r"(1) : "memory");
+	atomicExch(status, code);
+}
+__device__ __noinline__ bool dc_wait_slow(uint32_t base, uint32_t bar, uint32_t parity) {
+	return __all_sync(0xffffffffu, !dc_aborted(base) && mbar_wait_bounded(base + bar, parity, DC_SPIN));
+}
+__device__ __forceinline__ bool dc_wait(uint32_t base, uint32_t bar, uint32_t parity) {
+	return __all_sync(0xffffffffu, mbar_try_wait(base + bar, parity)) || dc_wait_slow(base, bar, parity);
 }
 __device__ __forceinline__ bool dc_elect() {
 	uint32_t r;
@@ -86,6 +102,25 @@ __device__ __forceinline__ uint32_t dc_lds16(uint32_t addr) {
 	asm volatile("ld.shared.u16 %0, [%1];" : "=h"(r) : "r"(addr) : "memory");
 	return r;
 }
+// Eight weights of a column, k order, as (q - zero) / 512 in fp16: exact (the nibble as a subnormal fp16 is q * 2^-24).
+template <int J>
+__device__ __forceinline__ uint32_t dc_pair(uint32_t e, uint32_t o, uint32_t zc) {
+	uint32_t r;          // bytes: even nibble, 0, odd nibble, 0 (selectors above 7 repeat a sign bit, which is zero)
+	asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(e), "r"(o), "n"(J | (8 + J) << 4 | (4 + J) << 8 | (12 + J) << 12));
+	return h2_fma(r, 0x78007800u, zc);
+}
+__device__ __forceinline__ void dc_unpack(uint32_t w, uint32_t zc, uint32_t *out) {
+	const uint32_t e = w & 0x0F0F0F0Fu, o = (w >> 4) & 0x0F0F0F0Fu;
+	out[0] = dc_pair<0>(e, o, zc);
+	out[1] = dc_pair<1>(e, o, zc);
+	out[2] = dc_pair<2>(e, o, zc);
+	out[3] = dc_pair<3>(e, o, zc);
+}
+__device__ __forceinline__ void dc_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+				 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+				 : "memory");
+}
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 	uint32_t *r = reinterpret_cast<uint32_t *>(v);
 	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -93,7 +128,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 				 : "r"(taddr)
 				 : "memory");
 }
-__device__ __forceinline__ void dc_workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DC_WORKERS) : "memory"); }
+// the NT threads that finish a tile
+template <int NT>
+__device__ __forceinline__ void dc_sync() { asm volatile("bar.sync %0, %1;" ::"n"(NT == DC_WORKERS ? 1 : 2), "n"(NT) : "memory"); }
 
 // Four partial sums of `count` CTAs, `stride` floats apart, added in order of K; four CTAs' values in flight.  Out of line: its registers
 // are not the main loop's.
@@ -118,8 +155,8 @@ __device__ __noinline__ float4 dec_gather(const float *src, int count, size_t st
 }
 
 // A tile's sums of this CTA (in shared memory, one part per group): handed over to the next CTA, or finished.
-template <int EPI, bool M8>
-__device__ __forceinline__ void dec_finish(const DecParams &p, const float *red, int tile, int k0, bool handed_over, int wid, volatile int *s_abort) {
+template <int EPI, bool M8, int NT>
+__device__ __forceinline__ void dec_finish(const DecParams &p, const float *red, int tile, int k0, bool handed_over, int wid, uint32_t base) {
 	constexpr bool PAIR = (EPI == DEC_EPI_SILU);
 	constexpr int TN = PAIR ? 64 : 128, ROWS = M8 ? 8 : 16;
 	const DecArgs &a = p.a;
@@ -140,29 +177,27 @@ __device__ __forceinline__ void dec_finish(const DecParams &p, const float *red,
 	if (handed_over) {
 		// the tile goes on in the next CTA's range, which finishes it
 		float4 *out = reinterpret_cast<float4 *>(p.partial + (size_t)cta * a.M * 128);
-		for (int e = wid; e < a.M * 32; e += DC_WORKERS) __stcg(out + e, own(e >> 5, (e & 31) * 4));
-		__threadfence();
-		dc_workers_sync();
+		for (int e = wid; e < a.M * 32; e += NT) __stcg(out + e, own(e >> 5, (e & 31) * 4));
+		dc_sync<NT>();                              // (the release below covers what it orders)
 		if (wid == 0) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p.flags + cta), "r"(1) : "memory");
 	} else {
 		int c0 = cta;                               // first CTA with a share of this tile
 		if (k0 > 0) {
 			while (c0 > 0 && first_unit(c0) > tile * np) --c0;
 			const unsigned long long t0 = global_timer_ns();
-			for (int c = c0 + wid; c < cta; c += DC_WORKERS) {
+			for (int c = c0 + wid; c < cta; c += NT) {
 				int f = 0;
 				for (;;) {
 					asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(f) : "l"(p.flags + c) : "memory");
 					if (f) break;
-					if (*s_abort || global_timer_ns() - t0 > 2000000000ull) {          // (bounded in time)
-						*s_abort = 1;
-						atomicExch(p.status, 6);
+					if (dc_aborted(base) || global_timer_ns() - t0 > 2000000000ull) {          // (bounded in time)
+						dc_abort(base, p.status, 6);
 						break;
 					}
 				}
 				p.flags[c] = 0;          // clean for the next launch
 			}
-			dc_workers_sync();
+			dc_sync<NT>();
 		}
 		auto sum = [&](int row, int col) {
 			const float4 s = own(row, col);
@@ -182,7 +217,7 @@ __device__ __forceinline__ void dec_finish(const DecParams &p, const float *red,
 		};
 		const int n0 = tile * TN;
 		if (EPI == DEC_EPI_PLAIN) {
-			for (int e = wid; e < a.M * 32; e += DC_WORKERS) {          // a warp has one row
+			for (int e = wid; e < a.M * 32; e += NT) {          // a warp has one row
 				const int row = e >> 5, col = (e & 31) * 4;
 				float4 v = sum(row, col);
 				if (a.bias) add4(v, a.bias + n0 + col);
@@ -198,7 +233,7 @@ __device__ __forceinline__ void dec_finish(const DecParams &p, const float *red,
 				}
 			}
 		} else if (EPI == DEC_EPI_SILU) {
-			for (int e = wid; e < a.M * 16; e += DC_WORKERS) {
+			for (int e = wid; e < a.M * 16; e += NT) {
 				const int row = e >> 4, col = (e & 15) * 4;
 				const float4 v = sum(row, col), u = sum(row, col + 64);
 				*reinterpret_cast<uint2 *>(a.y + (size_t)row * a.ldy + n0 + col) =
@@ -206,7 +241,7 @@ __device__ __forceinline__ void dec_finish(const DecParams &p, const float *red,
 			}
 		} else {
 			const int section = n0 / a.hidden, head = (n0 - section * a.hidden) >> 7;
-			for (int e = wid; e < a.M * 16; e += DC_WORKERS) {
+			for (int e = wid; e < a.M * 16; e += NT) {
 				const int row = e >> 4, d = (e & 15) * 4;
 				int pos = a.pos[row];
 				if (pos < 0 || pos >= a.max_pos) {          // never index the tables / the cache out of range
@@ -247,157 +282,162 @@ __device__ __forceinline__ void dec_finish(const DecParams &p, const float *red,
 	}
 }
 
-// x: warp xw stages the units xw, xw + 4, ...; lane -> eight k of every other row.  Out of line like the epilogue: a spilled register in
-// a loop costs an L2 round trip here (shared memory takes all of the L1).
-template <int EPI, bool M8>
-__device__ __noinline__ void dec_stage_x(const DecParams &p, int xw, int lane, uint32_t sX, uint32_t bar_full, uint32_t bar_done, float *s_inv, volatile int *s_abort) {
+// What a warp keeps between two tile segments.
+struct DecGroup {
+	int ws;                      // stage of the packed ring of its group's next unit
+	uint32_t wp, ph;             // phases of that stage and of the unit's stage in tensor memory
+	int st;                      // that stage
+	bool ok;
+};
+
+// One group's units of a tile segment (`count` of them): unpacked into tensor memory, their sums scaled and added, the tile's sums left in
+// shared memory, a part per group.  A store to tensor memory and its wait take longer than the unpacking of the words that it holds, so a
+// unit is only waited for, and handed to the MMAs, when the first words of the next one have been unpacked.
+template <bool PAIR, bool M8>
+__device__ __forceinline__ void dec_segment(uint32_t base, uint32_t tmem, int count, DecGroup &g, float *red, uint32_t red_empty, uint32_t red_parity) {
 	constexpr int ROWS = M8 ? 8 : 16;
-	const DecArgs &a = p.a;
-	const int np = a.K >> 7;
-	auto first_unit = [&](int c) { return (int)((long long)c * p.units / (int)gridDim.x); };
-	const int lo = first_unit(blockIdx.x), hi = first_unit(blockIdx.x + 1), n = hi - lo;
-	auto fail = [&](int code) {
-		*s_abort = 1;
-		atomicExch(p.status, code);
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = (warp - 8) >> 2, wt = (warp & 3) * 32 + lane;      // tensor-memory lane = weight column of the tile
+	constexpr uint32_t W_ROW = PAIR ? 256 : 512;
+	const uint32_t w_off = base + DC_OFF_W + (PAIR ? (uint32_t)((wt >> 6) * 4096 + (wt & 63) * 4) : (uint32_t)(wt * 4));
+	const uint32_t sc_off = base + DC_OFF_W + DC_W_SC + wt * 2, qz_off = base + DC_OFF_W + DC_W_QZ + (wt >> 3) * 4;
+	const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+	float acc[ROWS];
+#pragma unroll
+	for (int r = 0; r < ROWS; ++r) acc[r] = 0.f;
+	float sc0 = 0.f, sc1 = 0.f, sc2 = 0.f;          // scales of the unit in hand and of the two before
+	uint32_t zc = 0, w[16];
+	auto fetch = [&]() {
+		const uint32_t o = g.ws * DC_W_STAGE;
+		g.ok = g.ok && dc_wait(base, DC_FULL_W + 8 * g.ws, g.wp);
+		if (!g.ok) return;
+#pragma unroll
+		for (int r = 0; r < 16; ++r) w[r] = dc_lds32(w_off + o + r * W_ROW);
+		sc0 = 512.f * __half2float(__ushort_as_half((unsigned short)dc_lds16(sc_off + o)));
+		const uint32_t zz = ((dc_lds32(qz_off + o) >> ((wt & 7) * 4)) & 0xFu) + 1u;
+		zc = h2_mul(h2_sub((0x6400u + zz) * 0x00010001u, MAGIC_1024), 0x98009800u);      // half2(-zero / 512)
 	};
-	const int u = lane & 15, r0 = lane >> 4;
-	pdl_wait();
-	// behind the wait: what ran before this kernel is complete when its successor starts; not at all when it stores several cache rows of a
-	// sequence (see common.cuh)
-	if (EPI != DEC_EPI_ROPE || a.tokens_per_batch == 1) pdl_trigger();
-	const bool rms = EPI != DEC_EPI_PLAIN && a.rms_w != nullptr;
-	if (rms) {
-		// 1 / rms of every row from the per-tile sums the producing kernel left (fixed order)
-		for (int r = xw; r < a.M; r += 4) {
-			float v = 0.f;
-			for (int i = lane; i < a.ss_tiles; i += 32) v += __ldcg(a.ss_in + (size_t)r * a.ss_tiles + i);
-#pragma unroll
-			for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-			if (lane == 0) s_inv[r] = rsqrtf(v / (float)a.K + a.rms_eps);
-		}
-		asm volatile("bar.sync 2, 128;" ::: "memory");
-	}
-	constexpr int H = ROWS / 2;
-	const __half *src = a.x + (size_t)r0 * a.ldx + u * 8;
-	const size_t step = (size_t)2 * a.ldx;
-	uint4 v[H], wq;
-	int tile = (hi - 1) / np, k0 = max(lo - tile * np, 0), begin = 0, end = min(hi - tile * np, np) - k0;
-	auto load = [&](int i) {
-		while (i >= end) {                              // the segment that holds unit i
-			--tile;
-			k0 = max(lo - tile * np, 0);
-			begin = end;
-			end += np - k0;
-		}
-		const int k = (k0 + i - begin) * 128;
-#pragma unroll
-		for (int h = 0; h < H; ++h)
-			if (r0 + 2 * h < a.M) v[h] = __ldcg(reinterpret_cast<const uint4 *>(src + h * step + k));
-		if (rms) wq = __ldg(reinterpret_cast<const uint4 *>(a.rms_w + k + u * 8));
+	auto other = [&](int st) { return st >= DC_GROUPS ? st - DC_GROUPS : st + DC_GROUPS; };
+	auto hand_over = [&](int st) {                  // a unit's weights have landed
+		tmem_st_wait();
+		tc_fence_before();
+		__syncwarp();
+		if (lane == 0) mbar_arrive(base + DC_FULL + 8 * st);
 	};
-	if (xw < n) load(xw);
-	int s = xw;
-	uint32_t ph = 1;
-	for (int i = xw; i < n; i += 4) {
-		if (!dc_wait(bar_done + 8 * s, ph, s_abort)) { fail(3); break; }
-		const uint32_t dst = sX + s * DC_X_STAGE + (u >> 3) * 2048;
+	auto add = [&](int st, float scale) {           // a stage's sums: tensor memory -> registers
 #pragma unroll
-		for (int h = 0; h < H; ++h) {
-			const int row = r0 + 2 * h;
-			if (row < a.M) {
-				uint4 x = v[h];
-				if (rms) {
-					// x * inv_rms * w: fp32 product, one fp16 rounding (same expression as rmsnorm_kernel)
-					const float inv = s_inv[row];
-					const uint32_t xv[4] = {x.x, x.y, x.z, x.w}, wv[4] = {wq.x, wq.y, wq.z, wq.w};
-					uint32_t ov[4];
+		for (int h = 0; h < ROWS; h += 8) {
+			float d[8];
+			tmem_ld8(ta + st * DC_STAGE_COLS + DC_A_COLS + h, d);
+			tmem_ld_wait();
 #pragma unroll
-					for (int e = 0; e < 4; ++e) {
-						const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&xv[e])), g = __half22float2(*reinterpret_cast<const __half2 *>(&wv[e]));
-						const __half2 o = __floats2half2_rn(f.x * inv * g.x, f.y * inv * g.y);
-						ov[e] = *reinterpret_cast<const uint32_t *>(&o);
-					}
-					x = make_uint4(ov[0], ov[1], ov[2], ov[3]);
-				}
-				const uint32_t at = dst + (row >> 3) * 1024 + (row & 7) * 128 + (((u & 7) ^ (row & 7)) << 4);
-				asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(__byte_perm(x.x, x.z, 0x5410)), "r"(__byte_perm(x.x, x.z, 0x7632)),
-							 "r"(__byte_perm(x.y, x.w, 0x5410)), "r"(__byte_perm(x.y, x.w, 0x7632))
-							 : "memory");
+			for (int r = 0; r < 8; ++r) {
+				asm volatile("" : "+f"(d[r]));              // not before the wait
+				acc[h + r] = fmaf(scale, d[r], acc[h + r]);
 			}
 		}
-		fence_proxy_async();                            // (no load of this warp is in flight that it would wait for)
+	};
+	if (count > 0) fetch();
+#pragma unroll 1
+	for (int i = 0; i < count && g.ok; ++i) {
+		uint32_t o[16];
+#pragma unroll
+		for (int r = 0; r < 4; ++r) dc_unpack(w[r], zc, o + 4 * r);
+		if (i > 0) hand_over(other(g.st));
+		g.ok = dc_wait(base, DC_DONE + 8 * g.st, g.ph ^ 1);          // the unit that used this stage has been multiplied
+		if (!g.ok) break;
+		tc_fence_after();
+		const uint32_t at = ta + g.st * DC_STAGE_COLS;
+		dc_st16(at, o);
+#pragma unroll
+		for (int b = 1; b < 4; ++b) {
+			uint32_t v[16];
+#pragma unroll
+			for (int r = 0; r < 4; ++r) dc_unpack(w[4 * b + r], zc, v + 4 * r);
+			dc_st16(at + 16 * b, v);
+		}
 		__syncwarp();
-		if (lane == 0) mbar_arrive(bar_full + 8 * s);
-		if (i + 4 < n) load(i + 4);
-		s += 4;
-		if (s >= DC_STAGES) {
-			s -= DC_STAGES;
-			ph ^= 1;
+		if (lane == 0) mbar_arrive(base + DC_EMPTY_W + 8 * g.ws);
+		g.ws += DC_GROUPS;
+		if (g.ws >= DC_W_RING) {
+			g.ws -= DC_W_RING;
+			g.wp ^= 1;
+		}
+		if (i >= 2) add(g.st, sc2);                 // (an earlier segment's sums have been read)
+		sc2 = sc1;
+		sc1 = sc0;
+		if (i + 1 < count) fetch();
+		g.st += DC_GROUPS;
+		if (g.st >= DC_STAGES) {
+			g.st -= DC_STAGES;
+			g.ph ^= 1;
 		}
 	}
-	__syncwarp();
+	if (g.ok && count > 0) {
+		// the last two units: the next one's stage holds the older of them
+		hand_over(other(g.st));
+		if (count > 1) {
+			g.ok = dc_wait(base, DC_DONE + 8 * g.st, g.ph ^ 1);
+			tc_fence_after();
+			if (g.ok) add(g.st, sc2);
+		}
+		g.ok = g.ok && dc_wait(base, DC_DONE + 8 * other(g.st), g.st >= DC_GROUPS ? g.ph : g.ph ^ 1);
+		tc_fence_after();
+		if (g.ok) add(other(g.st), sc1);
+	}
+	tc_fence_before();
+	g.ok = g.ok && dc_wait(base, red_empty, red_parity);          // the tile two segments back has left the buffer
+#pragma unroll
+	for (int r = 0; r < ROWS; ++r) red[(grp * ROWS + r) * 128 + wt] = acc[r];
 }
 
 template <int EPI, bool M8>
 __global__ void __launch_bounds__(DC_THREADS, 1) dec_kernel(const __grid_constant__ CUtensorMap tmw0, const __grid_constant__ CUtensorMap tmw1,
-															const __grid_constant__ DecParams p) {
+															const __grid_constant__ CUtensorMap tmx, const __grid_constant__ DecParams p) {
 	extern __shared__ __align__(1024) unsigned char smem[];
-	__shared__ float s_inv[16];
 	constexpr bool PAIR = (EPI == DEC_EPI_SILU);             // 64 gate and 64 up columns per tile
-	constexpr int TN = PAIR ? 64 : 128, ROWS = M8 ? 8 : 16;
+	constexpr int TN = PAIR ? 64 : 128;
 	const DecArgs &a = p.a;
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x;
+	const int tid = threadIdx.x, warp = tid >> 5, cta = blockIdx.x;
 	const int np = a.K >> 7;
 	auto first_unit = [&](int c) { return (int)((long long)c * p.units / (int)gridDim.x); };
 	const int lo = first_unit(cta), hi = first_unit(cta + 1), n = hi - lo;
-
-	const uint32_t sX = smem_u32(smem), sW = sX + DC_OFF_W;
-	float *red = reinterpret_cast<float *>(smem + DC_OFF_RED);
-	uint64_t *bars = reinterpret_cast<uint64_t *>(smem + DC_OFF_BAR);
-	const uint32_t bar_full = smem_u32(bars), bar_done = bar_full + 8 * DC_STAGES, bar_full_w = bar_done + 8 * DC_STAGES, bar_empty_w = bar_full_w + 8 * DC_W_RING;
-	const uint32_t bar_fin = bar_empty_w + 8 * DC_W_RING;
-	uint32_t *s_tmem = reinterpret_cast<uint32_t *>(bars + 2 * DC_STAGES + 2 * DC_W_RING + 1);
-	volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
+	const uint32_t base = smem_u32(smem);
 
 	if (tid == 0) {
 		for (int s = 0; s < DC_STAGES; ++s) {
-			mbar_init(bar_full + 8 * s, 5);                   // four warps that unpack, one that stages x
-			mbar_init(bar_done + 8 * s, 1);                   // the unit's MMAs: sums are there, A and B are free
+			mbar_init(base + DC_FULL + 8 * s, 5);             // four warps that unpack, rows of x
+			mbar_init(base + DC_DONE + 8 * s, 1);             // sums are there, A and B are free
 		}
 		for (int s = 0; s < DC_W_RING; ++s) {
-			mbar_init(bar_full_w + 8 * s, 2);                 // words; scales and zeros
-			mbar_init(bar_empty_w + 8 * s, 4);
+			mbar_init(base + DC_FULL_W + 8 * s, 2);           // words; scales and zeros
+			mbar_init(base + DC_EMPTY_W + 8 * s, 4);
 		}
-		mbar_init(bar_fin, 1);
-		*s_abort = 0;
+		for (int s = 0; s < 2; ++s) {
+			mbar_init(base + DC_FULL_R + 8 * s, DC_WORKERS / 32);
+			mbar_init(base + DC_EMPTY_R + 8 * s, DC_FINISHERS / 32);
+		}
+		mbar_init(base + DC_FIN, 1);
+		*reinterpret_cast<volatile int *>(smem + DC_ABORT) = 0;
 		fence_mbar_init();
 		tma_prefetch_desc(&tmw0);
 		if (PAIR) tma_prefetch_desc(&tmw1);
+		tma_prefetch_desc(&tmx);
 	}
-	if (warp == 2) {
-		tmem_alloc(smem_u32(s_tmem), DC_TMEM_COLS);
+	if (warp == 1) {
+		tmem_alloc(base + DC_TMEM_ADDR, DC_TMEM_COLS);
 		tmem_relinquish();
 	}
-	// rows that do not exist are zero for good
-	for (int u = tid; u < DC_STAGES * DC_X_STAGE / 16; u += DC_THREADS) reinterpret_cast<uint4 *>(smem)[u] = make_uint4(0u, 0u, 0u, 0u);
-	fence_proxy_async();
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
-	const uint32_t tmem_a = *s_tmem, tmem_d = tmem_a + DC_STAGES * 64;
+	const uint32_t tmem = *reinterpret_cast<uint32_t *>(smem + DC_TMEM_ADDR);
 
-	auto fail = [&](int code) {
-		*s_abort = 1;
-		atomicExch(p.status, code);
-	};
 	if (warp == 0 || warp == 3) {
 		// ---------------- packed weights (warp 0), scales and zeros (warp 3); they depend on no earlier kernel ----------------
-		// Two warps, and nothing but additions per unit: with one warp and a division the chain of these instructions was the bound
-		// (8192 -> 16384, 16 rows: 25.0 us; without the division 22.0).
+		// Two warps, and nothing but additions per unit: with one warp and a division the chain of these instructions was the bound.
 		const int nz = a.N >> 3, gk = a.groupsize >> 7;
 		int s = 0, tile = (hi - 1) / np, left = n;
-		uint32_t ph = 1, dst = sW, bar = bar_full_w;
-		const uint32_t to_empty = bar_empty_w - bar_full_w;
+		uint32_t ph = 1, dst = base + DC_OFF_W, bar = DC_FULL_W;
 		const bool one = dc_elect();
 		bool ok = true;
 		while (left > 0 && ok) {
@@ -409,20 +449,20 @@ __global__ void __launch_bounds__(DC_THREADS, 1) dec_kernel(const __grid_constan
 			left -= len;
 			--tile;
 			for (int i = 0; i < len; ++i) {
-				ok = dc_wait(bar + to_empty, ph, s_abort);
+				ok = dc_wait(base, bar + (DC_EMPTY_W - DC_FULL_W), ph);
 				if (!ok) break;
 				if (one) {
 					if (warp == 0) {
-						mbar_arrive_expect_tx(bar, DC_W_SC);
-						tma_load_2d(dst, &tmw0, n0, row, bar);
-						if (PAIR) tma_load_2d(dst + 4096, &tmw1, n0, row, bar);
+						mbar_arrive_expect_tx(base + bar, DC_W_SC);
+						tma_load_2d(dst, &tmw0, n0, row, base + bar);
+						if (PAIR) tma_load_2d(dst + 4096, &tmw1, n0, row, base + bar);
 					} else {
-						mbar_arrive_expect_tx(bar, DC_W_BYTES - DC_W_SC);
-						dc_bulk_load(dst + DC_W_SC, sc0, TN * 2, bar);
-						dc_bulk_load(dst + DC_W_QZ, qz0, TN / 2, bar);
+						mbar_arrive_expect_tx(base + bar, DC_W_BYTES - DC_W_SC);
+						dc_bulk_load(dst + DC_W_SC, sc0, TN * 2, base + bar);
+						dc_bulk_load(dst + DC_W_QZ, qz0, TN / 2, base + bar);
 						if (PAIR) {
-							dc_bulk_load(dst + DC_W_SC + 128, sc1, TN * 2, bar);
-							dc_bulk_load(dst + DC_W_QZ + 32, qz1, TN / 2, bar);
+							dc_bulk_load(dst + DC_W_SC + 128, sc1, TN * 2, base + bar);
+							dc_bulk_load(dst + DC_W_QZ + 32, qz1, TN / 2, base + bar);
 						}
 					}
 				}
@@ -441,33 +481,70 @@ __global__ void __launch_bounds__(DC_THREADS, 1) dec_kernel(const __grid_constan
 				bar += 8;
 				if (++s == DC_W_RING) {
 					s = 0;
-					dst = sW;
-					bar = bar_full_w;
+					dst = base + DC_OFF_W;
+					bar = DC_FULL_W;
 					ph ^= 1;
 				}
 			}
 		}
 		if (!ok) {
-			fail(1);
+			dc_abort(base, p.status, 1);
 			const unsigned long long t0 = global_timer_ns();          // copies in flight land before the CTA may end
 			while (global_timer_ns() - t0 < 1000000ull) __nanosleep(1000);
 		}
+	} else if (warp == 2) {
+		// ---------------- rows of x: 16 rows x 128 k per unit, rows that do not exist are filled with zeros ----------------
+		const bool one = dc_elect();
+		pdl_wait();
+		// behind the wait: what ran before this kernel is complete when its successor starts; not at all when it stores several cache rows of a
+		// sequence (see common.cuh)
+		if (EPI != DEC_EPI_ROPE || a.tokens_per_batch == 1) pdl_trigger();
+		int s = 0, tile = (hi - 1) / np, left = n;
+		uint32_t ph = 1;
+		bool ok = true;
+		while (left > 0 && ok) {
+			const int k0 = max(lo - tile * np, 0), len = min(hi - tile * np, np) - k0;
+			left -= len;
+			--tile;
+			for (int k = k0 * 128; k < (k0 + len) * 128; k += 128) {
+				ok = dc_wait(base, DC_DONE + 8 * s, ph);
+				if (!ok) break;
+				if (one) {
+					const uint32_t bar = base + DC_FULL + 8 * s, dst = base + s * DC_X_BYTES;
+					mbar_arrive_expect_tx(bar, DC_X_BYTES);
+					tma_load_2d(dst, &tmx, k, 0, bar);
+					tma_load_2d(dst + DC_X_BYTES / 2, &tmx, k + 64, 0, bar);
+				}
+				__syncwarp();
+				if (++s == DC_STAGES) {
+					s = 0;
+					ph ^= 1;
+				}
+			}
+		}
+		if (!ok) {
+			dc_abort(base, p.status, 1);
+			const unsigned long long t0 = global_timer_ns();
+			while (global_timer_ns() - t0 < 1000000ull) __nanosleep(1000);
+		}
 	} else if (warp == 1) {
-		// ---------------- MMA issuer ----------------
+		// ---------------- MMA issuer: eight K = 16 steps per unit ----------------
 		const uint32_t idesc = (1u << 4) | ((uint32_t)(16 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);   // D fp32, A/B fp16 K-major, N = 16, M = 128
-		uint64_t xd = smem_desc_sw128(sX);
+		const uint64_t xd = smem_desc_sw128(base);
 		uint32_t ph = 0;
 		int s = 0;
 		const bool one = dc_elect();
+		bool ok = true;
 		for (int i = 0; i < n; ++i) {
-			if (!dc_wait(bar_full + 8 * s, ph, s_abort)) { fail(3); break; }
+			ok = dc_wait(base, DC_FULL + 8 * s, ph);
+			if (!ok) break;
 			tc_fence_after();
 			if (one) {
-				const uint32_t d = tmem_d + s * DC_D_COLS, at = tmem_a + s * 64;
-				const uint64_t xs = xd + (uint64_t)(s * (DC_X_STAGE >> 4));
+				const uint32_t at = tmem + s * DC_STAGE_COLS, d = at + DC_A_COLS;
+				const uint64_t xs = xd + (uint64_t)(s * (DC_X_BYTES >> 4));
 #pragma unroll
 				for (int k = 0; k < 8; ++k) umma_f16_ts(d, at + 8 * k, xs + (uint64_t)((k >> 2) * 128 + 2 * (k & 3)), idesc, k ? 1u : 0u);
-				umma_commit(bar_done + 8 * s);
+				umma_commit(base + DC_DONE + 8 * s);
 			}
 			__syncwarp();
 			if (++s == DC_STAGES) {
@@ -475,104 +552,56 @@ __global__ void __launch_bounds__(DC_THREADS, 1) dec_kernel(const __grid_constan
 				ph ^= 1;
 			}
 		}
-		if (one) umma_commit(bar_fin);
+		if (!ok) dc_abort(base, p.status, 3);
+		if (one) umma_commit(base + DC_FIN);
 		__syncwarp();
-	} else if (warp >= 4 && warp < 8) {
-		// ---------------- x ----------------
-		dec_stage_x<EPI, M8>(p, warp - 4, lane, sX, bar_full, bar_done, s_inv, s_abort);
-	} else if (warp >= 8) {
-		// ---------------- unpack, scale and add, epilogue ----------------
-		const int q = warp & 3, grp = (warp - 8) >> 2, wt = q * 32 + lane, wid = tid - 256;      // tensor-memory lane = weight column of the tile
-		const uint32_t w_off = PAIR ? (uint32_t)((wt >> 6) * 4096 + (wt & 63) * 4) : (uint32_t)(wt * 4);
-		constexpr uint32_t W_ROW = PAIR ? 256 : 512;
-		const uint32_t zsh = (wt & 7) * 4, quarter = (uint32_t)(q * 32) << 16;
-		bool ok = true, waited = false;
-		int i = grp, ws = grp;                              // next unit of this group, its stage of the packed ring
-		uint32_t wp = 0;
-		int tile = (hi - 1) / np, end = 0;                  // units of the segments so far
-		while (end < n) {
-			const int begin = end, k0 = max(lo - tile * np, 0), k1 = min(hi - tile * np, np);
+	} else if (warp < 8) {
+		// ---------------- finish every tile segment but the last one, while the next is unpacked ----------------
+		float *red = reinterpret_cast<float *>(smem + DC_OFF_RED);
+		int tile = (hi - 1) / np, b = 0;
+		uint32_t ph = 0;
+		pdl_wait();                                         // outputs, residual and the exchange area belong to earlier kernels until here
+		for (; tile * np > lo; --tile) {
+			if (!dc_wait(base, DC_FULL_R + 8 * b, ph)) break;
+			dec_finish<EPI, M8, DC_FINISHERS>(p, red + b * (DC_RED / 4), tile, 0, hi < (tile + 1) * np, tid - 128, base);
+			dc_sync<DC_FINISHERS>();
+			if ((tid & 31) == 0) mbar_arrive(base + DC_EMPTY_R + 8 * b);
+			b ^= 1;
+			ph ^= b == 0;
+		}
+	} else {
+		// ---------------- unpack, scale and add; finish the last segment ----------------
+		float *red = reinterpret_cast<float *>(smem + DC_OFF_RED);
+		int tile = (hi - 1) / np, end = 0, next = (warp - 8) >> 2, b = 0;      // units of the segments so far; next unit of this warp's group
+		uint32_t ph = 1;
+		DecGroup g = {next, 0u, 0u, next, true};
+		for (;; --tile) {
+			const int k0 = max(lo - tile * np, 0), k1 = min(hi - tile * np, np);
 			end += k1 - k0;
-			float acc[ROWS];
-#pragma unroll
-			for (int r = 0; r < ROWS; ++r) acc[r] = 0.f;
-			float sc1 = 0.f, sc2 = 0.f;                     // scales of the group's last unit and of the one before
-			// sums of unit v (its stage, phase): tensor memory -> registers
-			auto drain = [&](int v, float scale) {
-				const int st = v % DC_STAGES;
-				ok = ok && dc_wait(bar_done + 8 * st, (v / DC_STAGES) & 1, s_abort);
-				if (!ok) return;
-				tc_fence_after();
-				float d[ROWS];
-				if constexpr (M8) tmem_ld8(tmem_d + st * DC_D_COLS + quarter, d);
-				else tmem_ld16(tmem_d + st * DC_D_COLS + quarter, d);
-				tmem_ld_wait();
-#pragma unroll
-				for (int r = 0; r < ROWS; ++r) {
-					asm volatile("" : "+f"(d[r]));              // not before the wait
-					acc[r] = fmaf(scale, d[r], acc[r]);
-				}
-			};
-			for (; i < end && ok; i += DC_GROUPS) {
-				ok = dc_wait(bar_full_w + 8 * ws, wp, s_abort);
-				if (!ok) break;
-				if (i - DC_STAGES >= begin) drain(i - DC_STAGES, sc2);          // (an earlier segment's units have been drained)
-				if (!ok) break;
-				const uint32_t st = sW + ws * DC_W_STAGE, at = tmem_a + (i % DC_STAGES) * 64 + quarter;
-				sc2 = sc1;
-				sc1 = __half2float(__ushort_as_half((unsigned short)dc_lds16(st + DC_W_SC + wt * 2)));
-				const uint32_t zz = ((dc_lds32(st + DC_W_QZ + (wt >> 3) * 4) >> zsh) & 0xFu) + 1u;
-				const uint32_t ze = (0x6400u + zz) * 0x00010001u;            // half2(1024 + zero)
-				const uint32_t zo = (0xD400u + (zz << 4)) * 0x00010001u;     // half2(-(64 + zero))
-#pragma unroll
-				for (int h = 0; h < 2; ++h) {
-					uint32_t o[32];
-#pragma unroll
-					for (int r = 0; r < 8; ++r) {
-						const uint32_t w = dc_lds32(st + w_off + (8 * h + r) * W_ROW), w8 = w >> 8;
-						o[4 * r] = h2_sub(lop3_and_or(w, MASK_LO, MAGIC_1024), ze);                       // q - zero, exact: k0 k4
-						o[4 * r + 1] = h2_fma(lop3_and_or(w, MASK_HI, MAGIC_1024), 0x2C002C00u, zo);      // k1 k5
-						o[4 * r + 2] = h2_sub(lop3_and_or(w8, MASK_LO, MAGIC_1024), ze);                  // k2 k6
-						o[4 * r + 3] = h2_fma(lop3_and_or(w8, MASK_HI, MAGIC_1024), 0x2C002C00u, zo);     // k3 k7
-					}
-					tmem_st32(at + 32 * h, o);
-				}
-				__syncwarp();
-				if (lane == 0) mbar_arrive(bar_empty_w + 8 * ws);
-				tmem_st_wait();
-				tc_fence_before();
-				__syncwarp();
-				if (lane == 0) mbar_arrive(bar_full + 8 * (i % DC_STAGES));
-				ws += DC_GROUPS;
-				if (ws >= DC_W_RING) {
-					ws -= DC_W_RING;
-					wp ^= 1;
-				}
+			const int count = max(0, (end - next + DC_GROUPS - 1) / DC_GROUPS);
+			dec_segment<PAIR, M8>(base, tmem, count, g, red + b * (DC_RED / 4), DC_EMPTY_R + 8 * b, ph);
+			next += DC_GROUPS * count;
+			if (!g.ok) dc_abort(base, p.status, 3);
+			if (end >= n) {
+				pdl_wait();
+				dc_sync<DC_WORKERS>();
+				dec_finish<EPI, M8, DC_WORKERS>(p, red + b * (DC_RED / 4), tile, k0, k1 < np, tid - 256, base);
+				break;
 			}
-			if (i - 2 * DC_GROUPS >= begin) drain(i - 2 * DC_GROUPS, sc2);
-			if (i - DC_GROUPS >= begin) drain(i - DC_GROUPS, sc1);
-			tc_fence_before();
-			if (!ok) fail(3);
-#pragma unroll
-			for (int r = 0; r < ROWS; ++r) red[(grp * ROWS + r) * 128 + wt] = acc[r];
-			if (!waited) {
-				pdl_wait();                                 // outputs, residual and the exchange area belong to earlier kernels until here
-				waited = true;
-			}
-			dc_workers_sync();
-			dec_finish<EPI, M8>(p, red, tile, k0, k1 < np, wid, s_abort);
-			if (end < n) dc_workers_sync();                 // the tile in shared memory has been read
-			--tile;
+			__syncwarp();
+			if ((tid & 31) == 0) mbar_arrive(base + DC_FULL_R + 8 * b);
+			b ^= 1;
+			ph ^= b == 0;
 		}
 	}
 	tc_fence_before();
 	__syncthreads();
-	if (warp == 2) {
+	if (warp == 1) {
 		// tensor memory goes back only after every MMA issued above has completed (also when unwinding)
-		if (lane == 0) mbar_wait_bounded(bar_fin, 0, DC_SPIN);
+		if ((tid & 31) == 0) mbar_wait_bounded(base + DC_FIN, 0, DC_SPIN);
 		__syncwarp();
 		tc_fence_after();
-		tmem_dealloc(tmem_a, DC_TMEM_COLS);
+		tmem_dealloc(tmem, DC_TMEM_COLS);
 	}
 }
 
@@ -600,6 +629,19 @@ static int dec_map(const int32_t *qw, int K, int N, int cols, CUtensorMap *out) 
 	return GPTQ_OK;
 }
 
+// fp16 rows of x, boxes of 64 k x 16 rows, 128-byte swizzle
+static int dec_map_x(const DecArgs &a, CUtensorMap *out) {
+	cuuint64_t dims[2] = {(cuuint64_t)a.K, (cuuint64_t)a.M}, strides[1] = {(cuuint64_t)a.ldx * 2};
+	cuuint32_t box[2] = {64, 16}, estr[2] = {1, 1};
+	CUresult r = tensor_map_encoder()(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(a.x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+									  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+	if (r != CUDA_SUCCESS) {
+		g_last_cuda_error = (int)r;
+		return GPTQ_ERR_CUDA;
+	}
+	return GPTQ_OK;
+}
+
 template <int EPI, bool M8>
 static int dec_go(const DecParams &p, int grid, int dev, cudaStream_t stream) {
 	constexpr int TN = EPI == DEC_EPI_SILU ? 64 : 128;
@@ -610,11 +652,12 @@ static int dec_go(const DecParams &p, int grid, int dev, cudaStream_t stream) {
 		if (e != cudaSuccess) return cuda_status(e);
 		ready[dev] = true;
 	}
-	alignas(64) CUtensorMap tmw0, tmw1;
+	alignas(64) CUtensorMap tmw0, tmw1, tmx;
 	if (int rc = dec_map(p.a.qw0, p.a.K, p.a.N, TN, &tmw0)) return rc;
 	tmw1 = tmw0;
 	if (EPI == DEC_EPI_SILU)
 		if (int rc = dec_map(p.a.qw1, p.a.K, p.a.N, TN, &tmw1)) return rc;
+	if (int rc = dec_map_x(p.a, &tmx)) return rc;
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute attr[1];
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -625,7 +668,7 @@ static int dec_go(const DecParams &p, int grid, int dev, cudaStream_t stream) {
 	cfg.stream = stream;
 	cfg.attrs = attr;
 	cfg.numAttrs = pdl_enabled() ? 1 : 0;
-	return cuda_status(cudaLaunchKernelEx(&cfg, k, tmw0, tmw1, p));
+	return cuda_status(cudaLaunchKernelEx(&cfg, k, tmw0, tmw1, tmx, p));
 }
 
 int dec_launch(const DecArgs &a, int epi, void *workspace, size_t ws_bytes, cudaStream_t stream) {

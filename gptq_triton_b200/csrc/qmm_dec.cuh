@@ -20,11 +20,6 @@ struct DecArgs {
 	__half *y;
 	long long ldy;
 	float *ss_out;               // PLAIN: sums of squares of the outputs per 32 columns, or NULL
-	// x is RMS-normalised while it is staged
-	const __half *rms_w;
-	const float *ss_in;
-	int ss_tiles;
-	float rms_eps;
 	// ROPE
 	const __half *cos_t, *sin_t;
 	const int32_t *pos;

@@ -741,6 +741,37 @@ def test_decode_tensor_memory_kernel(G, K, gs, N, act, M):
 	assert _lib.kernel_status() == 0
 
 
+@pytest.mark.parametrize('M', [2, 8, 16])
+@pytest.mark.parametrize('K,N', [(128, 128 * 701), (384, 128 * 301), (1152, 128 * 148)])
+def test_decode_tensor_memory_kernel_many_tiles_per_cta(G, K, N, M):
+	"""Several tiles per CTA (four or five of one K-unit each, tiles that straddle CTAs, one whole tile each), rows of x that are further apart
+	than they are long, with NaN between them: every tile is finished beside the next one and the two buffers in between are used again."""
+	from gptq_triton_b200 import _lib
+	gs = 128
+	t, g, u = synth(K, N, gs, 1), synth(K, N // 2, gs, 2), synth(K, N // 2, gs, 3)
+	wide = torch.full((M, K + 24), float('nan'), dtype=torch.float16)
+	wide[:, :K] = acts((M, K), seed=4)
+	x, xd = wide[:, :K], wide.cuda()
+	norm_w = (1 + 0.1 * acts((1, K), seed=7).view(-1)).half()
+	xn = (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-6) * norm_w.float()).half()
+	ss = x.float().pow(2).view(M, K // 32, 32).sum(-1).contiguous().cuda()
+	y, h = torch.empty((M, N), dtype=torch.float16, device='cuda'), torch.empty((M, N // 2), dtype=torch.float16, device='cuda')
+	d = lambda w: [w[n].cuda() for n in ('qweight', 'qzeros', 'scales')]
+	P, st = _lib.ptr, _lib.stream_ptr(xd.device)
+	ws = _lib.workspace(xd.device, M, K, N)
+	td, gd, ud, wd = d(t), d(g), d(u), norm_w.cuda()
+	try:
+		_lib.lib().gptq_debug_dec_min_rows(1)
+		assert _lib.lib().gptq_qmatmul(P(xd), *map(P, td), None, None, None, None, N, P(y), M, K, N, gs, K + 24, N, P(ws), ws.numel(), st) == 0
+		assert _lib.lib().gptq_gateup_silu_rms(P(xd), *map(P, gd), *map(P, ud), None, None, P(h), M, K, N // 2, gs, K + 24, N // 2, P(ws), ws.numel(), st, P(wd), P(ss), K // 32, 1e-6) == 0
+		torch.cuda.synchronize()
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	assert O.max_rel_err(y, O.qmatmul_r32(x, t['qweight'], t['qzeros'], t['scales'], gs)) <= TOL
+	assert O.max_rel_err(h, O.gateup_silu_r32(xn, (g['qweight'], g['qzeros'], g['scales']), (u['qweight'], u['qzeros'], u['scales']), gs)) <= TOL
+	assert _lib.kernel_status() == 0 and not ws[:16384].any()
+
+
 @pytest.mark.parametrize('b', [1, 2])
 def test_attention_with_an_odd_number_of_keys(G, b):
 	"""QuantLlamaAttention with cached tokens and a mask whose rows do not start on 16 bytes, against its own path with explicit weights."""
