@@ -79,7 +79,7 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void *p) {
 // visible; nothing produced by an earlier kernel may be touched before it.
 // Read ahead of the wait all the same: weights, by every decode kernel; the position and old cache rows, by attn_decode_kernel (all but
 // the newest AT_FRESH) and qkv_attn_kernel.  A kernel that triggers BEFORE its own wait (skinny_kernel, attn_decode_kernel, qkv_attn_kernel,
-// rmsnorm_kernel, gather_x_kernel) hands the early start on: its successor may run while the kernel two launches back, if that one has
+// rmsnorm_kernel, norm_x_kernel, gather_x_kernel) hands the early start on: its successor may run while the kernel two launches back, if that one has
 // triggered too, is still storing.  So a kernel that stores several cache rows of a sequence does not trigger (its successor then starts behind
 // its last store): tc_kernel, which reads nothing ahead of its wait either, and the rotary forms of skinny_kernel and dec_kernel when a sequence has more than one
 // token.  dec_kernel otherwise triggers behind its wait, so that what ran before it is complete when its successor starts.
