@@ -18,6 +18,7 @@ _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / 'libgptq_b200.so'
 
 _lib: Optional[ctypes.CDLL] = None
+_host = None          # extension module csrc/host/calls.cpp, bound to the library
 
 _P = c_void_p
 _SIGNATURES = {
@@ -113,8 +114,21 @@ def lib() -> ctypes.CDLL:
 			l.gptq_debug_max_stages(int(os.environ['GPTQ_B200_STAGES']))      # ring depth of the decode kernel (A/B measurements)
 		if os.environ.get('GPTQ_B200_PDL', '1') == '0' and hasattr(l, 'gptq_debug_set_pdl'):
 			l.gptq_debug_set_pdl(0)      # opt out of programmatic dependent launch (A/B measurements)
-		_lib = l
+		try:
+			from . import _host as module
+		except ImportError as e:
+			raise ImportError(f'{_PKG / "_host.so"} is missing or does not fit this torch: build it with `python -m gptq_triton_b200.build`.') from e
+		address = lambda name: ctypes.cast(getattr(l, name), c_void_p).value
+		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope')))
+		_lib, globals()['_host'] = l, module
 	return _lib
+
+
+def host():
+	"""Layer calls in native code; each returns None when the call is not the plain case, and has then done nothing."""
+	if _host is None:
+		lib()
+	return _host
 
 
 class GptqB200Error(RuntimeError):
@@ -130,8 +144,7 @@ def check(code: int, what: str):
 		raise err(f'{what}: {msg}{extra}')
 
 
-# Addresses and streams go to ctypes as plain integers and the stream is asked for without building a Stream object: a call of the
-# smallest layer is bound by the host (o_proj of a 7B layer for one token: 27 us a call, 6 of them on the GPU).
+# Addresses and streams go to ctypes as plain integers and the stream is asked for without building a Stream object.
 def ptr(t: Optional[torch.Tensor]):
 	return None if t is None else t.data_ptr()
 

@@ -1,9 +1,10 @@
-"""Builds the in-tree C-ABI libraries with the sm_100a kernels with nvcc:
+"""Builds the in-tree C-ABI libraries with the sm_100a kernels with nvcc, and the extension module that calls them from Python:
 
   libgptq_b200.so    4-bit quantised linear layers, attention and decode kernels   (csrc/*.cu)
   libdense_b200.so   dense-weight layers and latent attention                      (csrc/dense/*.cu)
+  _host.so           layer calls without ctypes, against torch's C++ library       (csrc/host/*.cpp, with g++)
 
-Usage:  python -m gptq_triton_b200.build [--force] [--verbose] [gptq] [dense]
+Usage:  python -m gptq_triton_b200.build [--force] [--verbose] [gptq] [dense] [host]
 """
 from __future__ import annotations
 
@@ -12,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 from pathlib import Path
 from typing import Iterable, Optional
@@ -20,11 +22,13 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / 'csrc'
 LIB = PKG / 'libgptq_b200.so'
 DENSE_LIB = PKG / 'libdense_b200.so'
+HOST_LIB = PKG / '_host.so'
 
 # library -> (output, folder of its sources, further folders whose headers they include)
 TARGETS = {
 	'gptq': (LIB, CSRC, []),
 	'dense': (DENSE_LIB, CSRC / 'dense', [CSRC]),
+	'host': (HOST_LIB, CSRC / 'host', []),
 }
 
 NVCC_FLAGS = [
@@ -41,7 +45,15 @@ def _nvcc() -> str:
 
 
 def sources(target: str = 'gptq'):
-	return sorted(TARGETS[target][1].glob('*.cu'))
+	return sorted(TARGETS[target][1].glob('*.cpp' if target == 'host' else '*.cu'))
+
+
+def _host_command(out: str):
+	import torch
+	root = Path(torch.__file__).parent
+	paths = [f'-I{p}' for p in (root / 'include', Path(_nvcc()).resolve().parent.parent / 'include', sysconfig.get_paths()['include'])]
+	return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', *paths, '-o', out, *map(str, sources('host')),
+			f'-L{root / "lib"}', '-ltorch_python', '-ltorch_cpu', '-ltorch', '-lc10', '-lc10_cuda']
 
 
 def _fingerprint(target: str) -> str:
@@ -51,7 +63,11 @@ def _fingerprint(target: str) -> str:
 	for d in (folder, *more):
 		files += sorted(d.glob('*.cuh')) + sorted(d.glob('*.inl'))
 	files += sorted((PKG.parent / 'include').glob('*.h'))
-	h = hashlib.sha256(' '.join(NVCC_FLAGS).encode())
+	if target == 'host':
+		import torch
+		h = hashlib.sha256(f'{torch.__version__} {sys.version}'.encode())
+	else:
+		h = hashlib.sha256(' '.join(NVCC_FLAGS).encode())
 	for f in files:
 		h.update(f.name.encode())
 		h.update(f.read_bytes())
@@ -83,15 +99,16 @@ def _build_one(target: str, verbose: bool):
 	fd, part = tempfile.mkstemp(dir=PKG, prefix=f'.{out.stem}-', suffix='.so')      # a concurrent reader never sees half a library
 	os.close(fd)
 	try:
-		cmd = [_nvcc(), *NVCC_FLAGS, '-o', part, *map(str, sources(target))]
+		cmd = _host_command(part) if target == 'host' else [_nvcc(), *NVCC_FLAGS, '-o', part, *map(str, sources(target))]
 		if verbose:
-			cmd[1:1] = ['-Xptxas', '-v']
+			if target != 'host':
+				cmd[1:1] = ['-Xptxas', '-v']
 			print(' '.join(cmd))
 		r = subprocess.run(cmd, capture_output=True, text=True)
 		if verbose or r.returncode != 0:
 			sys.stderr.write(r.stdout + r.stderr)
 		if r.returncode != 0:
-			raise RuntimeError(f'nvcc failed building {out.name}')
+			raise RuntimeError(f'{Path(cmd[0]).name} failed building {out.name}')
 		os.chmod(part, 0o755)
 		os.replace(part, out)
 	finally:

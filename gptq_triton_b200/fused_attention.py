@@ -14,7 +14,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, quant_linear
 from .quant_linear import QuantLinear
 
 
@@ -50,6 +50,10 @@ def qkv_rope(groupsize: int, a: torch.Tensor, qweight, scales, qzeros, cos, sin,
 	assert qweight.shape[1] == 3 * hidden
 	pos = position_ids.reshape(-1).to(torch.int32).contiguous()
 	assert pos.numel() == M
+	if kv_cache is None and rms_weight is None:
+		out = _lib.host().qkv(_lib._workspaces, quant_linear.USE_TENSOR_CORE_KERNEL, groupsize, a, qweight, scales, qzeros, cos, sin, pos, n_heads, head_dim, perm)
+		if out is not None:
+			return out
 	# Q is written as [b, t, h, d]; the [b, h, t, d] view is returned
 	q = torch.empty((b, t, n_heads, head_dim), device=a.device, dtype=torch.float16)
 	if kv_cache is None:

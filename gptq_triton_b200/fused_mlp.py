@@ -12,8 +12,8 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from . import _lib
-from .quant_linear import QuantLinear
+from . import _lib, quant_linear
+from .quant_linear import QuantLinear, buffers
 
 
 def _is_llama_mlp(m) -> bool:
@@ -47,6 +47,10 @@ def gateup_silu(groupsize: int, a: torch.Tensor, gate_qweight, gate_scales, gate
 	RMS-normalised first: inside the decode kernel when `sumsq_in` (fp32 [M, K // 32], written by the
 	projection that produced `a`, see quant_linear.qmatmul) is given and the shape allows, else by the
 	library's RMSNorm kernel."""
+	if g_idx is None and rms_weight is None:
+		y = _lib.host().gateup(_lib._workspaces, quant_linear.USE_TENSOR_CORE_KERNEL, groupsize, a, gate_qweight, gate_scales, gate_qzeros, up_qweight, up_scales, up_qzeros, perm)
+		if y is not None:
+			return y
 	assert gate_qweight.shape == up_qweight.shape and gate_scales.shape == up_scales.shape and gate_qzeros.shape == up_qzeros.shape, "All weights must have the same shape"
 	assert a.shape[-1] == (gate_qweight.shape[0] * 8), "A must be a multiple of 8 in the last dimension"
 	assert a.is_contiguous(), "A must be contiguous"
@@ -148,8 +152,8 @@ class QuantLlamaMLP(nn.Module):
 	def intermediate(self, x, rms_weight=None, rms_eps=1e-6, sumsq_in=None):
 		if not self._ao_ready:
 			self._prepare()
-		return gateup_silu(self.groupsize, x, self._gate_qw, self.gate_proj_scales, self.gate_proj_qzeros,
-						   self._up_qw, self.up_proj_scales, self.up_proj_qzeros, g_idx=self._gidx, perm=self._perm,
+		gs, gz, us, uz = buffers(self, 'gate_proj_scales', 'gate_proj_qzeros', 'up_proj_scales', 'up_proj_qzeros')
+		return gateup_silu(self.groupsize, x, self._gate_qw, gs, gz, self._up_qw, us, uz, g_idx=self._gidx, perm=self._perm,
 						   rms_weight=rms_weight, rms_eps=rms_eps, sumsq_in=sumsq_in)
 
 	def forward(self, x, residual: Optional[torch.Tensor] = None, rms_weight=None, rms_eps=1e-6, sumsq_in=None, sumsq_out=None, ar=None):

@@ -61,6 +61,16 @@ def act_order_rows(qweight: torch.Tensor, perm: torch.Tensor) -> torch.Tensor:
 	return out
 
 
+def buffers(module: nn.Module, *names):
+	"""Attributes of a module that are buffers as a rule: looked up there first (half a microsecond less each than by attribute)."""
+	own = module._buffers
+	found = []
+	for name in names:
+		t = own.get(name)
+		found.append(getattr(module, name) if t is None else t)
+	return found
+
+
 DECODE_MAX_M = 16
 
 
@@ -100,6 +110,10 @@ def qmatmul(groupsize: int, a: torch.Tensor, qweight: torch.Tensor, scales: torc
 	projection; the partial sums of all ranks are added inside the kernel (every rank gets the
 	full result, residual included).
 	"""
+	if g_idx is None and sumsq_out is None and ar is None:
+		y = _lib.host().qmatmul(_lib._workspaces, USE_TENSOR_CORE_KERNEL, groupsize, a, qweight, scales, qzeros, bias, perm, residual)
+		if y is not None:
+			return y
 	assert a.shape[-1] == (qweight.shape[0] * 8), "A must be a multiple of 8 in the last dimension"
 	assert a.is_contiguous(), "A must be contiguous"
 	_lib.require_cuda(a, qweight, scales, qzeros, bias, g_idx, perm, residual)
@@ -266,9 +280,9 @@ class QuantLinear(nn.Module):
 			return self._ao_qweight, None, self._ao_perm
 		if self._ao_mode == 'general':
 			return self.qweight, self.g_idx, None
-		return self.qweight, None, None
+		return buffers(self, 'qweight')[0], None, None
 
 	def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None, sumsq_out: Optional[torch.Tensor] = None, ar=None) -> torch.Tensor:
 		qw, g_idx, perm = self.kernel_operands()
-		return qmatmul(self.groupsize, x, qw, self.scales, self.qzeros, self.bias, g_idx=g_idx, perm=perm, residual=residual,
-					   sumsq_out=sumsq_out, ar=ar)
+		scales, qzeros, bias = buffers(self, 'scales', 'qzeros', 'bias')
+		return qmatmul(self.groupsize, x, qw, scales, qzeros, bias, g_idx=g_idx, perm=perm, residual=residual, sumsq_out=sumsq_out, ar=ar)
