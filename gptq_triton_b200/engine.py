@@ -74,7 +74,7 @@ class StaticEngine:
 			self.tok.copy_(input_ids)
 			self.step()
 			# the graph's output tensor is overwritten by the next step
-			return self.logits.reshape(b, 1, -1)[:, [0] * len(want)].clone() if want else None
+			return self.logits.reshape(b, 1, -1).repeat(1, len(want), 1) if want else None          # (an index list would go to the device and wait for it)
 		order = sorted(range(len(want)), key=want.__getitem__)
 		parts = []
 		for lo in range(0, t, self.max_portion):
