@@ -62,6 +62,22 @@ def test_projection(control, dtype, M, K, N):
 	assert close(out[:, :N], 0.5 * ref, 2e-6)
 
 
+@pytest.mark.parametrize('M', [1, 5, 6])
+@pytest.mark.parametrize('K,N', [(16, 16), (64, 2368), (80, 2400), (528, 33), (2048, 7104), (5504, 2048), (11008, 64), (22016, 304)])
+def test_projection_of_few_rows(control, M, K, N):
+	"""Both sides of the limit of the kernel that streams through shared memory: less than a box of K, K slices that some warps have none of, one
+	tile more than SMs, several per CTA, rows that leave fewer stages; rows of x and of W further apart than they are long, NaN between."""
+	from gptq_triton_b200 import dense
+	gen = torch.Generator(device='cuda').manual_seed(K + N)
+	x, w = (torch.full((r, K + 24), float('nan'), device='cuda', dtype=B16) for r in (M, N))
+	x[:, :K], w[:, :K] = torch.randn((M, K), generator=gen, device='cuda').to(B16), torch.randn((N, K), generator=gen, device='cuda').to(B16)
+	x, w = x[:, :K], w[:, :K]
+	got = [dense.linear(x, w, control) for _ in range(3)]
+	ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+	assert ((got[0][:, :N] - ref).abs() <= 2.0 ** -24 * K * size).all()          # products are exact, K fp32 sums in some order
+	assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 @pytest.mark.parametrize('dtype', [F32, B16])
 @pytest.mark.parametrize('M', [1, 2, 3, 8, 40, 200])
 def test_mlp_sublayer(control, dtype, M):
