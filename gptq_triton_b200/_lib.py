@@ -63,6 +63,9 @@ _SIGNATURES = {
 	'gptq_qmatmul_noalloc': (c_int, [_P, _P, _P, _P, _P, _P, _P, c_int64, _P, c_int, c_int, c_int, c_int, c_int64, c_int64, _P]),
 	'gptq_noalloc_scratch_bytes': (c_size_t, [c_int, c_int, c_int, c_int]),
 	'gptq_noalloc_status': (c_int, [c_int]),
+	'gptq_attn_prompt_scratch_bytes': (c_size_t, [c_int, c_int, c_int]),
+	'gptq_attn_prompt_prepare': (c_int, [_P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, _P, c_int64, c_int64, _P, c_int64, c_int64, c_int, _P, _P, _P, c_size_t, _P]),
+	'gptq_attn_prompt': (c_int, [_P, c_int64, c_int64, c_int64, _P, _P, _P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, ctypes.c_float, _P, _P, c_size_t, _P]),
 	'gptq_chain_supported': (c_int, [c_int, c_int, c_int, c_int, c_int]),
 	'gptq_chain_desc_bytes': (c_size_t, [c_int]),
 	'gptq_chain_scratch_bytes': (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
@@ -119,7 +122,8 @@ def lib() -> ctypes.CDLL:
 		except ImportError as e:
 			raise ImportError(f'{_PKG / "_host.so"} is missing or does not fit this torch: build it with `python -m gptq_triton_b200.build`.') from e
 		address = lambda name: ctypes.cast(getattr(l, name), c_void_p).value
-		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope')))
+		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes',
+									 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')))
 		_lib, globals()['_host'] = l, module
 	return _lib
 

@@ -206,6 +206,18 @@ class QuantLlamaAttention(nn.Module):
 						position_ids, self.num_heads, self.head_dim, perm=perm, kv_cache=kv_cache, rms_weight=rms_weight, rms_eps=rms_eps,
 						sumsq_in=sumsq_in)
 
+	def _masked(self, hidden_states, mask, position_ids, past, need: int):
+		"""(output of the attention before o_proj, keys, values) from the kernels of csrc/attn_prompt.cu and the projection between them, or
+		None when the call is not their plain case (csrc/host/calls.cpp)."""
+		qw, g_idx, perm = self.qkv_proj.kernel_operands()
+		if g_idx is not None or past is not None and len(past) != 2:
+			return None
+		cos, sin = self.tables(hidden_states.device, need)
+		scales, qzeros = quant_linear.buffers(self.qkv_proj, 'scales', 'qzeros')
+		pk, pv = (None, None) if past is None else past
+		return _lib.host().attend(_lib._workspaces, quant_linear.USE_TENSOR_CORE_KERNEL, self.qkv_proj.groupsize, hidden_states, qw, scales, qzeros, cos, sin, position_ids,
+								  self.num_heads, perm, mask, pk, pv)
+
 	def forward(self, hidden_states: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
 				position_ids: Optional[torch.LongTensor] = None, past_key_value: Optional[Tuple[torch.Tensor]] = None,
 				output_attentions: bool = False, use_cache: bool = False
@@ -217,6 +229,11 @@ class QuantLlamaAttention(nn.Module):
 		past = 0 if past_key_value is None else past_key_value[0].shape[-2]
 		if position_ids is None:
 			position_ids = torch.arange(past, past + q_len, device=hidden_states.device).unsqueeze(0).expand(bsz, q_len)
+		if attention_mask is not None and not output_attentions and self.head_dim == 128:
+			served = self._masked(hidden_states, attention_mask, position_ids, past_key_value, past + q_len)
+			if served is not None:
+				out, key_states, value_states = served
+				return self.o_proj(out), None, (key_states, value_states) if use_cache else None
 		query_states, key_states, value_states = self.project_qkv(hidden_states, position_ids, need_positions=past + q_len)
 		if past_key_value is not None:
 			key_states = torch.cat([past_key_value[0], key_states], dim=2)

@@ -230,6 +230,22 @@ int gptq_embed_rmsnorm(const void *table, int64_t ldt, int64_t n_rows, const int
                        gptq_stream_t stream);
 
 /*
+ * Attention of a prompt behind cached tokens with an additive fp16 mask, head size 128 (the reference concatenates the cache and runs
+ * matmul / softmax / matmul, fused_attention.py:105-146).  mask: element strides mask_sb, mask_st, 1 of [mask_b, t, S], mask_b = b or 1 (shared).
+ *   gptq_attn_prompt_prepare   classifies the tiles of the mask into `scratch` and copies the `past` cached rows (element strides per sequence
+ *                              and head, rows of 128) to the front of k, v [b, heads, S, 128]
+ *   gptq_attn_prompt           out [b, t, heads * 128] = softmax(q k^T scale + mask) v; a query that sees nothing gets zeros.  scratch NULL:
+ *                              no tile of the mask has been classified
+ */
+size_t gptq_attn_prompt_scratch_bytes(int b, int t, int S);
+int gptq_attn_prompt_prepare(const void *mask, int64_t mask_sb, int64_t mask_st, int mask_b, int b, int heads, int t, int S,
+                             const void *past_k, int64_t pk_sb, int64_t pk_sh, const void *past_v, int64_t pv_sb, int64_t pv_sh,
+                             int past, void *k, void *v, void *scratch, size_t scratch_bytes, gptq_stream_t stream);
+int gptq_attn_prompt(const void *q, int64_t q_sb, int64_t q_st, int64_t q_sh, const void *k, const void *v, const void *mask,
+                     int64_t mask_sb, int64_t mask_st, int mask_b, int b, int heads, int t, int S, float scale, void *out,
+                     const void *scratch, size_t scratch_bytes, gptq_stream_t stream);
+
+/*
  * RMSNorm folded into the decode kernels (M <= 16).  No counterpart in the reference, whose
  * decoder layer runs the HF LlamaRMSNorm module between its fused ops.  A decode step otherwise
  * spends two extra launches per layer on the norm; here the projection that produces the

@@ -1,0 +1,131 @@
+"""Attention of a prompt behind cached tokens with an additive mask: the kernels against 64 bits, and the calls of the attention block that run on
+them against the path that they replace."""
+
+import pytest
+import torch
+
+import gptq_triton_b200 as G
+from gptq_triton_b200 import _lib, synth
+
+pytestmark = pytest.mark.gpu
+INF = float('inf')
+
+
+def _mask(kind, b, t, S, gen):
+	past = S - t
+	hidden = torch.triu(torch.ones((t, S), dtype=torch.bool, device='cuda'), diagonal=past + 1)
+	m = torch.zeros((b, 1, t, S), device='cuda', dtype=torch.float16)
+	if kind == 'shared':
+		return m[:1].masked_fill(hidden, -INF).expand(b, 1, t, S)
+	if kind == 'lowest':
+		return m.masked_fill(hidden, torch.finfo(torch.float16).min)
+	if kind == 'random':
+		return torch.randn((b, 1, t, S), generator=gen, device='cuda').half()
+	if kind == 'padded':          # every sequence hides a different number of leading keys, and its first queries see nothing at all
+		for i in range(b):
+			m[i, :, :, :(i * 37) % S] = -INF
+			m[i, :, :min(i, t)] = -INF
+		return m.masked_fill(hidden, -INF)
+	wide = torch.zeros((b, 1, t, S + 5), device='cuda', dtype=torch.float16)          # rows that start anywhere
+	wide[..., 3:S + 3] = m.masked_fill(hidden, -INF)
+	return wide[..., 3:S + 3]
+
+
+@pytest.mark.parametrize('kind', ['shared', 'lowest', 'random', 'padded', 'wide'])
+@pytest.mark.parametrize('b,H,t,past', [(1, 2, 1, 5), (3, 2, 7, 0), (2, 3, 64, 64), (1, 2, 65, 63), (3, 2, 130, 1), (2, 1, 63, 200), (1, 2, 300, 128)])
+def test_kernels(kind, b, H, t, past):
+	gen = torch.Generator(device='cuda').manual_seed(t)
+	S, D = t + past, 128
+	rnd = lambda *shape: torch.randn(shape, generator=gen, device='cuda').half()
+	q, new_k, new_v, mask = rnd(b, t, H, D), rnd(b, H, t, D), rnd(b, H, t, D), _mask(kind, b, t, S, gen)
+	old_k, old_v = rnd(b, H, past + 3, D)[:, :, :past], rnd(b, past, H, D).transpose(1, 2).contiguous()
+	k, v = (torch.full((b, H, S, D), float('nan'), dtype=torch.float16, device='cuda') for _ in range(2))
+	k[:, :, past:], v[:, :, past:] = new_k, new_v
+	mask_b = 1 if mask.stride(0) == 0 else b
+	need = _lib.lib().gptq_attn_prompt_scratch_bytes(mask_b, t, S)
+	flags = torch.full((need + 64,), 7, dtype=torch.uint8, device='cuda')
+	P, st = _lib.ptr, _lib.stream_ptr(q.device)
+	where = (P(mask), mask.stride(0), mask.stride(2), mask_b, b, H, t, S)
+	assert _lib.lib().gptq_attn_prompt_prepare(*where, P(old_k), *old_k.stride()[:2], P(old_v), *old_v.stride()[:2], past, P(k), P(v), P(flags), need, st) == 0
+	whole_k, whole_v = torch.cat([old_k, new_k], 2), torch.cat([old_v, new_v], 2)
+	assert torch.equal(k, whole_k) and torch.equal(v, whole_v) and bool((flags[:need] < 3).all()) and bool((flags[need:] == 7).all())
+	outs = []
+	for scratch, size in ((flags, need), (None, 0)):
+		out = torch.full((b, t, H * D), float('nan'), dtype=torch.float16, device='cuda')
+		rc = _lib.lib().gptq_attn_prompt(P(q), t * H * D, H * D, D, P(k), P(v), *where[:4], b, H, t, S, D ** -0.5, P(out), P(scratch), size, st)
+		assert rc == 0
+		outs.append(out.view(b, t, H, D).transpose(1, 2))
+	s = q.transpose(1, 2).double() @ whole_k.double().transpose(2, 3) * D ** -0.5 + mask.double()
+	ref = torch.softmax(s, -1).nan_to_num(0.0) @ whole_v.double()          # a query that sees nothing: zeros
+	# weights and result are rounded to fp16 (2^-11 of at most max |v| each); the rest is fp32
+	bound = 1.1 * 2.0 ** -10 * float(whole_v.abs().max())
+	for out in outs:
+		assert float((out.double() - ref).abs().max()) <= bound
+
+
+def test_what_the_mask_holds():
+	"""A row of infinities or NaN makes its own query NaN, nothing else; refused sizes and alignments come back as errors."""
+	b, H, t, S, D = 1, 2, 70, 134, 128
+	q, k, v = (torch.randn(b, n, H, D, device='cuda').half() for n in (t, S, S))
+	k, v = k.transpose(1, 2).contiguous(), v.transpose(1, 2).contiguous()
+	mask = torch.zeros((b, 1, t, S), device='cuda', dtype=torch.float16)
+	mask[0, 0, 3], mask[0, 0, 68] = INF, float('nan')
+	out = torch.empty((b, t, H * D), dtype=torch.float16, device='cuda')
+	P, st = _lib.ptr, _lib.stream_ptr(q.device)
+	f = _lib.lib().gptq_attn_prompt
+	assert f(P(q), t * H * D, H * D, D, P(k), P(v), P(mask), t * S, S, 1, b, H, t, S, D ** -0.5, P(out), None, 0, st) == 0
+	bad = out.isnan().all(-1)[0]
+	assert bad[3] and bad[68] and int(out.isnan().any(-1).sum()) == 2
+	assert f(None, 0, 0, 0, P(k), P(v), P(mask), t * S, S, 1, b, H, t, S, 1.0, P(out), None, 0, st) == -1
+	assert f(P(q), t * H * D, H * D, D, P(k), P(v), P(mask), t * S, S, 2, b, H, t, S, 1.0, P(out), None, 0, st) == -1
+	assert f(P(q), t * H * D, H * D + 4, D, P(k), P(v), P(mask), t * S, S, 1, b, H, t, S, 1.0, P(out), None, 0, st) == -4
+
+
+@pytest.mark.parametrize('b,t,past,kind,served', [(1, 1, 40, 'shared', True), (2, 9, 0, 'shared', True), (1, 140, 61, 'lowest', True), (2, 33, 96, 'padded', True), (1, 201, 64, 'wide', True),
+												  (1, 2040, 8, 'shared', True), (1, 2048, 8, 'shared', False), (1, 3000, 0, 'shared', False), (1, 3001, 0, 'shared', True), (2, 33, 96, 'float32', False),
+												  (2, 33, 96, 'bool', False), (1, 33, 0, 'grad', False), (1, 33, 30, 'transposed past', False)])
+def test_calls_of_the_block(monkeypatch, b, t, past, kind, served):
+	H, K = 2, 256
+	def layer(N, seed):
+		d = synth.quant_tensors(K, N, 128, seed)
+		q = G.QuantLinear(4, 128, K, N, False)
+		q.qweight, q.qzeros, q.scales = d['qweight'], d['qzeros'], d['scales']
+		return q
+	attn = G.QuantLlamaAttention(G.LlamaConfig(hidden_size=K, num_attention_heads=H, max_position_embeddings=4096), layer(3 * K, 1), layer(K, 2), None).cuda()
+	gen = torch.Generator(device='cuda').manual_seed(5)
+	x = torch.randn((b, t, K), generator=gen, device='cuda').half()
+	kv = tuple(torch.randn((b, H, past, 128), generator=gen, device='cuda').half() for _ in range(2)) if past else None
+	mask = _mask(kind if kind in ('shared', 'lowest', 'padded', 'wide') else 'shared', b, t, past + t, gen)
+	if kind == 'float32':
+		mask = mask.float()
+	elif kind == 'bool':
+		mask = mask == 0
+	elif kind == 'grad':
+		mask = mask.clone().requires_grad_()
+	elif kind == 'transposed past':
+		kv = tuple(p.transpose(1, 2).contiguous().transpose(1, 2) for p in kv)
+	host, seen = _lib.host(), []
+
+	class Counts:
+		qmatmul, gateup, qkv = host.qmatmul, host.gateup, host.qkv
+		attend = staticmethod(lambda *a: seen.append(host.attend(*a)) or seen[-1])
+
+	class Declines(Counts):
+		attend = staticmethod(lambda *a: None)
+
+	def call(module):
+		with monkeypatch.context() as m:
+			m.setattr(_lib, '_host', module)
+			return attn(x, attention_mask=mask, past_key_value=kv, use_cache=True)
+	call(Declines)          # (the workspace is there)
+	new, old = call(Counts), call(Declines)
+	assert len(seen) == 1 and (seen[0] is not None) == served
+	assert new[1] is None and all(torch.equal(a, c) and a.stride() == c.stride() for a, c in zip(new[2], old[2]))
+	if served:
+		scale = float(old[0].float().abs().max())
+		assert float((new[0].float() - old[0].float()).abs().max()) <= 2e-3 * scale          # two roundings of the softmax weights
+	else:
+		assert torch.equal(new[0].nan_to_num(7.0), old[0].nan_to_num(7.0))
+	assert attn(x, attention_mask=mask, past_key_value=kv)[2] is None
+	with pytest.raises(ValueError):
+		attn(x, attention_mask=torch.zeros((b, 1, t, past + t + 1), device='cuda').half(), past_key_value=kv)

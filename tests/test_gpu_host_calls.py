@@ -46,7 +46,8 @@ def _layer(K, N, gs, bias=False, act=False, seed=1):
 
 
 @pytest.mark.parametrize('M,K,N,gs,bias,act', [(1, 256, 128, 128, False, False), (7, 512, 256, -1, True, False), (16, 1024, 384, 128, True, True), (17, 512, 256, 64, False, False),
-												(40, 1024, 256, 128, True, False), (3, 96, 40, 32, False, False)])
+												(40, 1024, 256, 128, True, False), (3, 96, 40, 32, False, False),
+												(40, 1024, 256, 128, False, True), (40, 256, 72, 32, True, False), (20, 256, 128, 32, False, True)])
 @pytest.mark.parametrize('residual', [False, True])
 def test_linear(monkeypatch, M, K, N, gs, bias, act, residual):
 	layer = _layer(K, N, gs, bias, act)
@@ -58,9 +59,12 @@ def test_linear(monkeypatch, M, K, N, gs, bias, act, residual):
 
 
 @pytest.mark.parametrize('M', [1, 16, 33])
-def test_mlp_and_qkv(monkeypatch, M):
+@pytest.mark.parametrize('gs,act', [(128, False), (32, False), (128, True)])
+def test_mlp_and_qkv(monkeypatch, M, gs, act):
 	H, I = 256, 384
-	mlp = G.QuantLlamaMLP(_layer(H, I, 128, seed=1), _layer(I, H, 128, seed=2), _layer(H, I, 128, seed=3))
+	gate, up = (_layer(H, I, gs, act=act, seed=s) for s in (1, 3))
+	up.set_g_idx(gate.g_idx)
+	mlp = G.QuantLlamaMLP(gate, _layer(I, H, gs, act=act, seed=2), up)
 	x = torch.randn(1, M, H, device='cuda').half()
 	attn = G.QuantLlamaAttention(G.LlamaConfig(hidden_size=H, num_attention_heads=2), _layer(H, 3 * H, 128, seed=4), _layer(H, H, 128, seed=5), None)
 	mlp(x), attn(x)
