@@ -3,7 +3,7 @@
 //
 // Grid (splits, heads, batch).  A CTA of 8 warps takes a contiguous range of cache positions and
 // pulls it into shared memory with bulk asynchronous copies (64 keys of K and of V per stage,
-// three stages, mbarrier completion).  The copies are issued BEFORE the kernel waits for its
+// two or three stages, mbarrier completion).  The copies are issued BEFORE the kernel waits for its
 // predecessor in the stream: old cache rows do not depend on it, so the cache streams in while
 // the QKV kernel of the same step is still finishing.  Only the newest AT_FRESH positions are
 // read from global memory after the wait (they may have been written by that kernel).
@@ -39,6 +39,7 @@ struct AttnParams {
 	long long out_stride_b;
 	float scale;
 	int heads, splits;
+	int stages;               // 2 or AT_STAGES
 	float *ws_partial;        // [b*heads][splits][130]
 	int *ws_ticket;           // [b*heads]
 };
@@ -49,7 +50,7 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint
 				 : "memory");
 }
 
-__global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(const AttnParams p) {
+__global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(const AttnParams p) {
 	extern __shared__ __align__(128) unsigned char at_smem[];
 	const int split = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -67,14 +68,15 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(const AttnParam
 	__shared__ float s_m[AT_GROUPS], s_l[AT_GROUPS];
 	float(*s_acc)[AT_D] = reinterpret_cast<float(*)[AT_D]>(at_smem);      // [AT_GROUPS][128], over the drained stages
 	__shared__ int s_last;
-	const uint32_t bar0 = smem_u32(at_smem + AT_STAGES * AT_STAGE_BYTES);
+	const int nst = p.stages;
+	const uint32_t bar0 = smem_u32(at_smem + nst * AT_STAGE_BYTES);
 	if (tid == 0) {
-		for (int s = 0; s < AT_STAGES; ++s) mbar_init(bar0 + 8 * s, 1);
+		for (int s = 0; s < nst; ++s) mbar_init(bar0 + 8 * s, 1);
 		fence_mbar_init();
 	}
 	__syncthreads();
-	auto issue = [&](int c) {                // one thread: K and V rows of chunk c into stage c % AT_STAGES
-		const int stage = c % AT_STAGES, key0 = k_lo + c * AT_CHUNK;
+	auto issue = [&](int c, int stage) {     // one thread: K and V rows of chunk c
+		const int key0 = k_lo + c * AT_CHUNK;
 		const uint32_t bytes = (uint32_t)min(AT_CHUNK, k_hi - key0) * AT_D * 2u;
 		const uint32_t dst = smem_u32(at_smem + stage * AT_STAGE_BYTES), bar = bar0 + 8 * stage;
 		mbar_arrive_expect_tx(bar, 2u * bytes);
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(const AttnParam
 		bulk_load_1d(dst + AT_STAGE_BYTES / 2, vbase + (size_t)key0 * AT_D, bytes, bar);
 	};
 	if (tid == 0)
-		for (int c = 0; c < min(nchunks, AT_STAGES); ++c) issue(c);
+		for (int c = 0; c < min(nchunks, nst); ++c) issue(c, c);
 	pdl_wait();                                          // q and the newest cache rows come from earlier kernels
 
 	// this lane's 16 query dims (sub*8 .. +7 and 64 + sub*8 .. +7), pre-scaled
@@ -109,10 +111,10 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(const AttnParam
 	constexpr int KPG = AT_CHUNK / AT_GROUPS;       // keys per 8-lane group and chunk
 	bool failed = false;
 #pragma unroll 1
-	for (int c = 0; c < nchunks; ++c) {
-		const int stage = c % AT_STAGES, key0 = k_lo + c * AT_CHUNK;
+	for (int c = 0, stage = 0, phase = 0; c < nchunks; ++c) {
+		const int key0 = k_lo + c * AT_CHUNK;
 		const int n = min(AT_CHUNK, k_hi - key0);
-		const bool got = mbar_wait_bounded(bar0 + 8 * stage, (c / AT_STAGES) & 1);
+		const bool got = mbar_wait_bounded(bar0 + 8 * stage, phase);
 		if (!__syncthreads_and(got)) {       // the same verdict for every thread
 			failed = true;
 			break;
@@ -167,9 +169,13 @@ __global__ void __launch_bounds__(AT_THREADS) attn_decode_kernel(const AttnParam
 				m = mn;
 			}
 		}
-		if (c + AT_STAGES < nchunks) {       // the stage is refilled once every thread has read it
+		if (c + nst < nchunks) {             // the stage is refilled once every thread has read it
 			__syncthreads();
-			if (tid == 0) issue(c + AT_STAGES);
+			if (tid == 0) issue(c + nst, stage);
+		}
+		if (++stage == nst) {
+			stage = 0;
+			phase ^= 1;
 		}
 	}
 	if (failed && tid == 0 && p.ws_ticket) atomicExch(p.ws_ticket + AT_STATUS_SLOT, 1);      // a bulk copy never completed

@@ -399,6 +399,24 @@ def test_attn_decode_matches_fp32_reference(G, b, heads, S, positions):
 	assert O.max_rel_err(out.view(b, -1), ref.float()) <= TOL
 
 
+@pytest.mark.parametrize('heads', [37, 38])
+def test_attn_decode_of_more_pairs_than_a_wave(G, heads):
+	"""Both sides of the line from which a CTA has two stages instead of three (8 sequences x 37 heads fit two CTAs per SM): lengths of one chunk of 64
+	keys to seven, so that stages are used up to four times."""
+	from gptq_triton_b200 import _lib
+	from gptq_triton_b200.fused_attention import attn_decode
+	b, S, D = 8, 448, 128
+	positions = torch.tensor([0, 63, 64, 127, 128, 200, 320, 447], dtype=torch.int32)
+	gen = torch.Generator(device='cuda').manual_seed(heads)
+	q, kc, vc = (torch.randn(shape, generator=gen, device='cuda').half() for shape in ((b, 1, heads, D), (b, heads, S, D), (b, heads, S, D)))
+	out = attn_decode(q.transpose(1, 2), kc, vc, positions.view(b, 1).cuda(), len_hint=S)
+	s = torch.einsum('bhd,bhsd->bhs', q[:, 0].double(), kc.double()) / D ** 0.5
+	s.masked_fill_(torch.arange(S, device='cuda')[None, None] > positions.cuda()[:, None, None], -float('inf'))
+	ref = torch.einsum('bhs,bhsd->bhd', torch.softmax(s, -1), vc.double()).reshape(b, -1)
+	assert O.max_rel_err(out.view(b, -1).cpu(), ref.float().cpu()) <= TOL
+	assert _lib.kernel_status() == 0
+
+
 @pytest.mark.parametrize('M,K', [(1, 4096), (5, 512), (16, 11008)])
 def test_rmsnorm_kernel(G, M, K):
 	from gptq_triton_b200.fused_attention import rmsnorm
