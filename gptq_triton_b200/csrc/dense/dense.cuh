@@ -144,11 +144,30 @@ __device__ __forceinline__ float rp_sqdev(float4 v, float mean, int c, int width
 	return s;
 }
 // (v - mean) * inv * gain + shift, gain and shift optional
-__device__ __forceinline__ float4 rp_affine(float4 v, float mean, float inv, const float *gain, const float *shift, int u) {
-	const float4 g = gain ? __ldg(reinterpret_cast<const float4 *>(gain) + u) : make_float4(1.f, 1.f, 1.f, 1.f);
-	const float4 s = shift ? __ldg(reinterpret_cast<const float4 *>(shift) + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+__device__ __forceinline__ float4 rp_gain(const float *gain, int u) { return gain ? __ldg(reinterpret_cast<const float4 *>(gain) + u) : make_float4(1.f, 1.f, 1.f, 1.f); }
+__device__ __forceinline__ float4 rp_shift(const float *shift, int u) { return shift ? __ldg(reinterpret_cast<const float4 *>(shift) + u) : make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ float4 rp_affine(float4 v, float mean, float inv, float4 g, float4 s) {
 	return make_float4(fmaf((v.x - mean) * inv, g.x, s.x), fmaf((v.y - mean) * inv, g.y, s.y), fmaf((v.z - mean) * inv, g.z, s.z), fmaf((v.w - mean) * inv, g.w, s.w));
 }
+__device__ __forceinline__ float4 rp_affine(float4 v, float mean, float inv, const float *gain, const float *shift, int u) { return rp_affine(v, mean, inv, rp_gain(gain, u), rp_shift(shift, u)); }
+
+// Weights and biases of both norms for the units that a thread keeps in registers.  They depend on no launch, but a step's weights have pushed them out of
+// L2 by the time they are wanted: fetched ahead of the dependency wait they are not a trip to HBM between the sums and the rows.
+struct RowWeights {
+	float4 gain[RP_REGS], shift[RP_REGS], w[RP_REGS], b[RP_REGS];
+	__device__ __forceinline__ void load(const RowPrep &p) {
+#pragma unroll
+		for (int i = 0; i < RP_REGS; ++i) {
+			const int u = threadIdx.x + i * DN_THREADS;
+			if (u < (p.ld >> 2)) {
+				gain[i] = rp_gain(p.gain, u);
+				shift[i] = rp_shift(p.shift, u);
+				w[i] = rp_gain(p.fin_w, u);
+				b[i] = rp_shift(p.fin_b, u);
+			}
+		}
+	}
+};
 
 // The RMS norm of equal parts of row x (global memory, `width` columns): a warp sums a share of a part, the shares of a part
 // are added in order.  inv: fin_groups (or DN_WARPS, if that is more) floats of shared memory.
@@ -233,8 +252,8 @@ __device__ void norm_parts(const RowPrep &p, const S *x, T *dst, float *inv) {
 
 // The whole CTA (256 threads) prepares one row.  dst: where the T row goes (global or shared memory); write_x: also store
 // the new residual row.  red: RP_SMEM floats of shared memory, reused across rows (callers synchronise between rows).
-template <typename T>
-__device__ void prepare_row(const RowPrep &p, int m, T *dst, bool write_x, float *red) {
+template <typename T, bool EARLY = false>
+__device__ void prepare_row(const RowPrep &p, int m, T *dst, bool write_x, float *red, const RowWeights *weights = nullptr) {
 	const int tid = threadIdx.x, nu = p.ld >> 2;
 	size_t xb = (size_t)m * p.ld, pb = 0;
 	const size_t yb = xb;
@@ -298,7 +317,7 @@ __device__ void prepare_row(const RowPrep &p, int m, T *dst, bool write_x, float
 	for (int i = 0; i < RP_REGS; ++i) {
 		const int u = tid + i * DN_THREADS;
 		if (u < nu) {
-			x[i] = next_x(x[i], y[i], u);
+			x[i] = EARLY ? (p.y ? add4(x[i], rp_affine(y[i], mean, inv, weights->gain[i], weights->shift[i])) : x[i]) : next_x(x[i], y[i], u);
 			if (write_x) reinterpret_cast<float4 *>(p.x_out + yb)[u] = x[i];
 			if (!norm) Elem<T>::store4(dst + 4 * u, x[i]);
 		}
@@ -330,7 +349,12 @@ __device__ void prepare_row(const RowPrep &p, int m, T *dst, bool write_x, float
 	for (int i = 0; i < RP_REGS; ++i) s += rp_sqdev(x[i], fm, 4 * (tid + i * DN_THREADS), p.width);
 	for (int u = tid + RP_REGS * DN_THREADS; u < nu; u += DN_THREADS) s += rp_sqdev(far_x(u), fm, 4 * u, p.width);
 	const float fi = 1.f / sqrtf(block_sum(s, red + 3 * DN_WARPS) * inv_n + p.eps);
-	for (int i = 0, u = tid; u < nu; ++i, u += DN_THREADS) {
+	if (EARLY) {
+#pragma unroll
+		for (int i = 0; i < RP_REGS; ++i)
+			if (tid + i * DN_THREADS < nu) Elem<T>::store4(dst + 4 * (tid + i * DN_THREADS), rp_affine(x[i], fm, fi, weights->w[i], weights->b[i]));
+	}
+	for (int i = EARLY ? RP_REGS : 0, u = tid + i * DN_THREADS; u < nu; ++i, u += DN_THREADS) {
 		float4 v;
 		if (i < RP_REGS) {
 			v = i == 0 ? x[0] : i == 1 ? x[1] : i == 2 ? x[2] : x[3];

@@ -275,6 +275,8 @@ __global__ void __launch_bounds__(DN_THREADS, 1) dense_ring_kernel(const __grid_
 	};
 #pragma unroll 1
 	for (int s = 0; s < stages; ++s) load();     // weights do not depend on earlier kernels
+	RowWeights weights;
+	if (p.prep) weights.load(p.rp);
 	pdl_wait();
 	pdl_trigger();
 
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(DN_THREADS, 1) dense_ring_kernel(const __grid_
 	if (p.prep) {
 		for (int m = 0; m < p.M; ++m) {
 			if (m) __syncthreads();
-			prepare_row<bf16>(p.rp, m, reinterpret_cast<bf16 *>(rows + (size_t)m * xs), p.rp.x_out != nullptr && blockIdx.x == 0, s_norm);
+			prepare_row<bf16, true>(p.rp, m, reinterpret_cast<bf16 *>(rows + (size_t)m * xs), p.rp.x_out != nullptr && blockIdx.x == 0, s_norm, &weights);
 		}
 	} else {
 		const int units = p.K / 8;
