@@ -5,7 +5,7 @@
 // holds the INTEGERS q - zero as fp16 (times 2^-9), which is exact; a unit of 128 K-rows lies in one group, so its fp32 sums leave tensor memory,
 // are multiplied with the group's scale in fp32 and added in registers.  No weight is rounded.
 //
-// Split of the work: one CTA per SM, fewer when there are less than two units for each; the units of all tiles (128 columns, or 64 gate + 64 up)
+// Split of the work: one CTA per SM (four SMs stay free, see dec_launch()), fewer when there are less than two units for each; the units of all tiles (128 columns, or 64 gate + 64 up)
 // x K / 128 are one list that is cut into ranges which differ by at most one unit of 128 x 128 weights.  A CTA walks its tiles from the last to the first: the tile
 // whose end lies in the next CTA's range comes first and its partial sums are handed over early, the tile whose beginning lies in the
 // ranges of earlier CTAs comes last and is finished there (partial sums added in order of K: deterministic).  A CTA only ever waits for
@@ -20,8 +20,8 @@
 // What bounds it: stores to tensor memory.  A unit is 32 KB of fp16 there and takes about 0.27 us (some 64 bytes a clock; without three quarters
 // of the stores, all else equal, 0.20 us a unit, which is what the weights take from HBM), and about 6 us from launch to exit (prologue, first
 // copies, hand-over).  Measured against the mma.sync kernel (qmm_skinny.cuh), us, 16 rows:
-//   4096 -> 4096 8.4 (11.5)   4096 -> 12288 12.9 (17.9)   11008 -> 4096 11.9 (18.4)   8192 -> 24576 29.4 (57.3)   22016 -> 8192 27.0 (55.4)
-//   gate/up 4096 -> 2 x 11008 18.0 (35.3)   8192 -> 2 x 22016 50 (110)
+//   4096 -> 4096 7.8 (11.5)   4096 -> 12288 12.2 (17.9)   11008 -> 4096 11.3 (18.4)   8192 -> 24576 29.3 (57.3)   22016 -> 8192 27.2 (55.4)
+//   gate/up 4096 -> 2 x 11008 17.5 (35.3)   8192 -> 2 x 22016 50 (110)
 // What brought it there (same sizes, before: 9.7, 13.8, 13.3, 31.6, 28.4, 21.6, 61): x by TMA instead of four warps that permuted it for every
 // unit (gate/up 61 -> 54), the norm in a kernel of its own (82.6 -> 58), tiles finished beside the main loop and a hand-over without a
 // fence per thread (4 us of each launch), stores to tensor memory in four parts that overlap with the unpacking (54 -> 50).  Eight warps per
@@ -55,7 +55,7 @@ constexpr int DC_FULL_R = DC_EMPTY_W + 8 * DC_W_RING, DC_EMPTY_R = DC_FULL_R + 1
 constexpr int DC_A_COLS = 64, DC_STAGE_COLS = DC_A_COLS + 16, DC_TMEM_COLS = 512;
 constexpr uint32_t DC_SPIN = 1u << 24;
 constexpr int DC_COUNTERS = 16384;                           // bytes of the workspace's counter area; its last word is the status word
-constexpr int DC_MAX_CTAS = 256;
+constexpr int DC_MAX_CTAS = 256, DC_SPARE = 4;
 static_assert(DC_STAGES * DC_STAGE_COLS <= DC_TMEM_COLS && DC_W_RING % DC_GROUPS == 0 && DC_STAGES % DC_GROUPS == 0, "rings");
 static_assert(DC_SMEM + 512 <= 227 * 1024, "shared memory per CTA");
 
@@ -684,7 +684,13 @@ int dec_launch(const DecArgs &a, int epi, void *workspace, size_t ws_bytes, cuda
 	p.partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(workspace) + DC_COUNTERS);
 	auto even = [](const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 7u) == 0; };
 	p.out8 = even(a.q_out) && even(a.k_out) && even(a.v_out) && ((a.q_stride_m | a.kv_sb | a.kv_st | a.kv_sh | a.kv_sp) & 3) == 0;
-	const int grid = std::max(1, std::min({sms, DC_MAX_CTAS, p.units / 2}));          // at least two units each
+	// At least two units per CTA, and four SMs left free: a CTA needs a whole SM, so with one on each SM the next launch's CTA starts only when the
+	// last one of this launch has left its SM, and the launch lasts as long as that one needs from its start (8.7 us where the others are done 5.3 us
+	// after their wait).  With SMs to spare every CTA of the next launch fills its ring beforehand.  148 / 147 / 144 / 140 CTAs, 16 rows, us:
+	// 4096 -> 4096 8.4 / 8.2 / 7.8 / 7.8, 4096 -> 12288 12.7 / 12.6 / 12.2 / 12.4, 8192 -> 24576 (83 units for each) 29.8 / 29.4 / 29.3 / 30.3; a decode
+	// step of 4 layers of 4096 355 -> 342.  From 100 units on the lost SMs weigh more: gate/up of 8192 -> 2 x 22016 (149 units) 50.1 / 50.2 / 50.8 / 51.8.
+	const int spare = sms > DC_SPARE && p.units < 100 * sms ? DC_SPARE : 0;
+	const int grid = std::max(1, std::min({sms - spare, DC_MAX_CTAS, p.units / 2}));
 	const bool m8 = a.M <= 8;
 	switch (epi) {
 		case DEC_EPI_PLAIN: return m8 ? dec_go<DEC_EPI_PLAIN, true>(p, grid, dev, stream) : dec_go<DEC_EPI_PLAIN, false>(p, grid, dev, stream);
