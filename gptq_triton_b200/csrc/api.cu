@@ -237,28 +237,35 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 	grid = dim3(tiles, p.splitk, 1);
 }
 
-// Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one; 17: never.  Its time hardly depends on the rows, its start and
-// end cost about 3 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows.  Measured in us, tensor
-// memory / this kernel (dependent launches, weights from HBM):
-//   4096 -> 4096 (8 MB)           M = 4   7.5 / 7.1    M = 7   7.6 / 9.6    M = 9   7.7 / 10.6   M = 16   8.4 / 11.5
-//   11008 -> 4096 (23 MB)         M = 4  10.9 / 11.3   M = 6  11.0 / 12.9   M = 9  11.3 / 17.2   M = 16  11.9 / 18.4
-//   4096 -> 12288 (25 MB)         M = 4  12.0 / 10.9   M = 5  12.1 / 12.3   M = 9  12.4 / 16.5   M = 16  12.9 / 17.9
-//   gate/up 4096 -> 2 x 11008     M = 3  17.5 / 17.3   M = 4  17.5 / 18.4   M = 8  17.6 / 24.1   M = 16  18.0 / 35.3
-//   22016 -> 8192 (90 MB)         M = 2  25.5 / 25.3   M = 3  25.5 / 27.9   M = 7  25.7 / 40.1   M = 16  27.0 / 55.4
-//   gate/up 8192 -> 2 x 11008     M = 2  27.2 / 26.9   M = 3  27.1 / 28.6   M = 8  27.2 / 38.3   M = 16  27.9 / 66.3
-//   8192 -> 24576 (101 MB)        M = 2  28.1 / 29.4   M = 4  28.1 / 33.8   M = 8  28.1 / 41.2   M = 16  29.4 / 57.3
-//   the same with the folded norm (a kernel of its own ahead of this one): gate/up 8192 -> 2 x 22016   M = 1  50.2 / 49.8   M = 2  51.4 / 54.2
-//   M = 16  53.7 / 119;   gate/up 4096 -> 2 x 11008   M = 3  18.4 / 18.2   M = 4  18.7 / 19.5   M = 16  19.7 / 38.0
+// Rows from which the tensor-memory kernel (qmm_dec.cu) is the faster one; 17: never.  Its time hardly depends on the rows; its start and
+// end cost some 2 us more than this kernel's, whose unpacking of a weight is followed by an MMA per eight rows and whose plan for more than four
+// rows has larger tiles of x.  Measured in us, tensor memory / this kernel (dependent launches, weights from HBM):
+//   4096 -> 4096 (8 MB)           M = 4   7.0 / 7.2    M = 5   7.1 / 8.5    M = 9   7.3 / 10.6   M = 16   7.8 / 11.5
+//   2048 -> 6144 (6 MB)           M = 4   6.9 / 7.2    M = 5   6.9 / 8.4    M = 9   7.0 / 9.9    M = 16   7.3 / 10.9
+//   11008 -> 4096 (23 MB)         M = 4  10.5 / 11.3   M = 5  10.5 / 12.2   M = 9  10.8 / 17.2   M = 16  11.4 / 18.4
+//   4096 -> 12288 (25 MB)         M = 4  11.8 / 10.8   M = 5  11.9 / 12.3   M = 9  12.0 / 16.7   M = 16  12.4 / 18.0
+//   8192 -> 8192 (34 MB)          M = 3  13.5 / 13.0   M = 4  13.6 / 13.3   M = 5  13.5 / 15.1   M = 16  14.6 / 21.5
+//   5120 -> 15360 (39 MB)         M = 3  15.4 / 15.1   M = 4  15.2 / 15.9   M = 5  15.2 / 17.6   M = 16  16.2 / 42.2
+//   22016 -> 8192 (90 MB)         M = 2  25.5 / 25.3   M = 3  25.6 / 27.9   M = 7  25.7 / 40.2   M = 16  26.9 / 55.4
+//   8192 -> 24576 (101 MB)        M = 2  27.7 / 29.4   M = 4  27.8 / 33.7   M = 8  27.9 / 41.2   M = 16  29.2 / 57.4
+// Gate and up (twice the MMAs there, the same work here); `norm`: the folded norm, a kernel of its own ahead of this one:
+//   1024 -> 2 x 2816              M = 2   7.0 / 7.4    M = 3   7.1 / 8.6    M = 16   7.1 / 16.4
+//   2048 -> 2 x 5504, norm        M = 2   9.5 / 9.7    M = 3   9.5 / 10.8   M = 16   9.9 / 21.7
+//   3072 -> 2 x 8192              M = 2  12.4 / 10.9   M = 3  12.5 / 12.4   M = 4   12.4 / 13.5   M = 16  12.9 / 24.8
+//   4096 -> 2 x 11008             M = 2  17.2 / 15.9   M = 3  17.2 / 17.3   M = 4   17.2 / 18.3   M = 16  17.8 / 35.2
+//   8192 -> 2 x 22016, norm       M = 1  50.1 / 49.8   M = 2  51.5 / 54.3   M = 16  53.9 / 119
 // A narrow layer with a deep K is the exception: every tile of 128 columns is spread over many CTAs, and the last one adds their sums.
-//   4096 -> 2048 (16 tiles)     M = 7   7.6 / 6.8    M = 9   7.7 / 8.4    M = 16  8.5 / 8.9
-//   8192 -> 1024 (8 tiles)      M = 7   9.8 / 8.4    M = 9   9.8 / 9.2    M = 16 11.7 / 9.7
-//   8192 -> 3072 (24 tiles)     M = 8   9.2 / 9.0    M = 9   9.4 / 11.3   M = 16 10.2 / 12.0
-//   2048 -> 2048 (16)           M = 4   5.0 / 4.5    M = 7   5.0 / 6.4
+//   4096 -> 2048 (16 tiles)       M = 5   6.5 / 6.3    M = 7   6.5 / 6.8    M = 16  7.6 / 8.8
+//   8192 -> 2048                  M = 4   7.5 / 5.8    M = 5   7.5 / 7.5    M = 16  8.6 / 10.5
+//   8192 -> 1024 (8 tiles)        M = 7   8.6 / 8.4    M = 9   8.8 / 9.2    M = 16 10.2 / 9.7
+// The lines of the layers of fewer than 48 tiles are those of an earlier form of the kernel, which took 1 us more; they are pinned by tests.
 static int dec_min_rows(int K, int N, int nstream, bool rope) {
 	const int tiles = N / 128;
 	if (nstream == 1 && tiles < 30 && (rope ? K >= 1536 : K > 2048)) return tiles <= 16 ? 17 : 9;
 	const double mb = (double)K * N * nstream / 2e6;
-	return mb >= 100 ? 2 : mb >= 64 ? 3 : mb >= 40 ? 4 : mb >= 24 ? 5 : mb >= 20 ? 6 : 7;
+	if (mb >= 100) return 2;
+	if (nstream == 2 || mb >= 64) return 3;
+	return mb >= 32 ? 4 : mb >= 24 || tiles >= 48 ? 5 : mb >= 20 ? 6 : 7;
 }
 
 // Narrow geometry (one 32-column strip and the whole of K per CTA, no split-K): worth it when

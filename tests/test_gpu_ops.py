@@ -888,6 +888,26 @@ def test_which_decode_kernel_runs(G, kind, K, N, M, tensor_memory):
 	assert torch.equal(outs[0], outs[1] if tensor_memory else outs[2])
 
 
+@pytest.mark.parametrize('pair,K,N,M,tensor_memory', [
+	(False, 2048, 6016, 6, False), (False, 2048, 6144, 4, False), (False, 2048, 6144, 5, True), (False, 6144, 10240, 4, False), (False, 6272, 10240, 4, True),
+	(True, 1024, 1024, 2, False), (True, 1024, 1024, 3, True), (True, 8192, 12160, 2, False), (True, 8192, 12288, 2, True)])
+def test_which_decode_kernel_runs_for_wide_and_paired_layers(G, pair, K, N, M, tensor_memory):
+	"""The same for layers of 48 tiles and more, and for gate and up."""
+	from gptq_triton_b200 import _lib
+	layers = [[v.cuda() for v in (t['qweight'], t['scales'], t['qzeros'])] for t in (synth(K, N, 128, seed) for seed in range(1 + pair))]
+	x = acts((1, M, K), seed=M).cuda()
+	outs = []
+	try:
+		for rows in (0, 1, 17):
+			_lib.lib().gptq_debug_dec_min_rows(rows)
+			outs.append(G.gateup_silu(128, x, *layers[0], *layers[1]) if pair else G.qmatmul(128, x, *layers[0]))
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	assert not torch.equal(outs[1], outs[2])
+	assert torch.equal(outs[0], outs[1] if tensor_memory else outs[2])
+	assert ((outs[1].float() - outs[2].float()).abs().max() / outs[2].float().abs().max()).item() <= 2 * TOL
+
+
 @pytest.mark.parametrize('M', [17, 40, 144, 145])
 @pytest.mark.parametrize('K,gs', [(192, 64), (448, 64), (192, 192)])
 def test_prefill_of_large_scales_behind_an_odd_number_of_k_blocks(G, M, K, gs):
