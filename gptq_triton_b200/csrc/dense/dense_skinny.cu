@@ -234,9 +234,11 @@ __global__ void __launch_bounds__(DN_THREADS, 2) dense_skinny_kernel(const Dense
 // tiles through a ring of its own (boxes of 16 rows x 64 k by TMA, 128-byte swizzle).  Five boxes of 2 KB for each of eight warps keep 80 KB in flight
 // per SM, twice what the registers hold, and the ring is full before the launch in front ends.
 // Bound: HBM for wide layers (32000 x 2048: 24.3 us = 5.4 TB/s alone), else the chain wait - rows - sums - store of about 4.5 us per launch.  In a step
-// (2048 hidden): down 9.2 -> 5.4 us, gate/up 13.0 -> 11.1, out 4.9 -> 4.6; the step 433 -> 400 us, of the state-space model 273 -> 251.
+// (2048 hidden): down 9.2 -> 5.4 us, gate/up 13.0 -> 11.1, out 4.9 -> 4.6; the step 433 -> 400 us, of the state-space model 273 -> 251, and with the norm weights ahead
+// of the wait (RowWeights) 381 and 240.
 // One CTA per SM, by the shared memory that it asks for: with two resident CTAs per SM, so that the next launch's rings could fill beside this
-// one, the scheduler puts two CTAs of one launch on some SMs and none on others (head 31 -> 67 us, step 482).  More stages are slower (10: 417).
+// one, the scheduler puts two CTAs of one launch on some SMs and none on others (head 31 -> 67 us, step 482).  More stages are slower (10: 417),
+// and SMs left free for the next launch change nothing (148 / 144 / 140 CTAs: 382 / 384 / 384; 3 layers of 4096 313 / 314 / 324).
 constexpr int RG_ROWS = 5, RG_STAGES = 5, RG_BOX = 2048, RG_MIN_SMEM = 120 * 1024;
 constexpr int RG_STATIC = (2 * DN_WARPS * SK_M * SK_REDLD + RP_SMEM) * (int)sizeof(float) + DN_WARPS * RG_STAGES * 8 + 64 + 1024;
 
@@ -386,8 +388,8 @@ int launch(const DenseArgs &a, cudaStream_t stream) {
 	int kparts = a.K * (int)sizeof(T) > 8192 ? SK_PARTS : 1;
 	while (kparts > 1 && (ntiles * kparts > dn_sm_count() || a.K < kparts * DN_WARPS * 64 / (int)sizeof(T))) kparts >>= 1;
 	if (kparts > 1 && !a.e.best && smem <= 160 * 1024) return dn_launch_as(kparts, -1, dense_skinny_kernel<T, true>, dim3(ntiles * kparts), dim3(DN_THREADS), smem, stream, a, kparts);
-	// Up to five rows: per decode step of a latent-attention model in us, this kernel / the one below: 8 layers of 2048 hidden, 1 row 400 / 433; 4 and
-	// 3 layers of 2048 and 4096, 2 rows 239 / 251 and 358 / 361, 5 rows 279 / 294 and 399 / 421; 8 rows 297 / 341 and 486 / 472 (there the rows
+	// Up to five rows: per decode step of a latent-attention model in us, this kernel / the one below: 8 layers of 2048 hidden, 1 row 381 / 433; 4 and
+	// 3 layers of 2048 and 4096, 2 rows 228 / 251 and 358 / 361, 5 rows 279 / 294 and 397 / 421; 8 rows 297 / 341 and 486 / 472 (there the rows
 	// of the widest layers do not fit, and every change between the two kernels' shared-memory splits costs more than the kernel gains).
 	if (sizeof(T) == 2 && a.M <= RG_ROWS)
 		if (const int stages = ring_stages(a)) return launch_ring(a, stages, stream);
