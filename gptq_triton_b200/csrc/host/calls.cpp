@@ -290,7 +290,7 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 		if (pk && (!head_rows(*pk, b, H) || !head_rows(*pv, b, H) || pv->size(2) != past)) return nullptr;
 		// Long prompts whose mask rows start on 16 bytes are better off with the library kernel.  Whole block, this kernel / library, us: 32 heads, t = 1000 198 / 169,
 		// t = 400 of 5 sequences 312 / 295, t = 200 56 / 65, t = 64 40 / 65, t = 2 behind 100 36 / 80; 16 heads, t = 1200 98 / 105.  Rows off 16 bytes have to be
-		// copied for it: t = 701 behind 64 124 / 159, t = 1300 241 / 318, t = 2048 behind 1500 588 / 677.
+		// copied for it: t = 701 behind 64 113 / 159, t = 1300 241 / 318, t = 2048 behind 1500 588 / 677.
 		const bool off = t > 128 && (mask->stride(2) % 8 != 0 || reinterpret_cast<uintptr_t>(mask->data_ptr()) % 16 != 0);
 		if (!off && b * H * t * S > (8 << 20)) return nullptr;
 		if (!c.workspace(a[0], w.K, w.N) || !c.gather(w, perm)) return nullptr;
