@@ -166,10 +166,12 @@ static int tc_map(const void *base, CUtensorMapDataType type, int elem, cuuint64
 constexpr int TC_MAX_SPLITS = 8;       // portable cluster size
 // Estimated time of a CTA in us, fitted to measurements (M = 17 .. 2048, K = 4096 / 8192 / 11008 / 22016): a K-block costs the
 // dequantisation (0.16 us at 32 rows in stages of two, 0.22 in stages of one) or the MMAs (0.38 us at 256 rows), a tile 2.5 us to start and
-// drain; with split K the partial tiles of the cluster are summed through distributed shared memory (4.8 us at 32 rows, 7 us at 256).
+// drain; with split K the partial tiles of the cluster are summed through distributed shared memory (4 us at 32 rows, 7 us at 256).  Against 4.8 us at 32
+// rows, a first fit on K >= 4096 only, us (dependent launches): 1024 -> 1024, 40 rows 5.9 -> 5.4; 2048 -> 6144, 17 rows 9.2 -> 8.4; 2048 -> 3072, 203 rows 10.1 -> 9.5;
+// 3072 -> 3072, 203 rows 11.4 -> 10.6; 2560 -> 7680, 100 rows 11.6 -> 10.7; 5504 -> 2048, 512 rows 16.6 -> 15.2; the wide layers choose as before.
 static double tc_cta_us(int nr, int splits, int kblocks) {
 	const double t_kb = nr <= TC_PAIR_NR ? 0.14 + 0.00065 * nr : std::max(0.22 + 0.0002 * nr, 0.0015 * nr);
-	return kblocks * t_kb + (splits > 1 ? 4.5 + 0.01 * nr : 2.5);
+	return kblocks * t_kb + (splits > 1 ? 3.5 + 0.014 * nr : 2.5);
 }
 
 template <int EPI, int KP>
