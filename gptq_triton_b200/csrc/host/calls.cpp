@@ -87,6 +87,7 @@ struct Call {
 	cudaStream_t stream = nullptr;
 	void *ws = nullptr;
 	size_t ws_bytes = 0;
+	at::Tensor held;          // the workspace: another thread may take it out of the table while the library runs without the GIL
 
 	bool input(PyObject *o) {
 		x = plain(o, at::kHalf, -1);
@@ -141,6 +142,7 @@ struct Call {
 		}
 		const at::Tensor *t = plain(found, at::kByte, device);
 		if (!t) return false;
+		held = *t;
 		ws = t->data_ptr();
 		ws_bytes = t->numel();
 		return ws_bytes >= workspace_bytes((int)M, (int)K, (int)N);

@@ -124,3 +124,33 @@ def test_what_is_not_the_plain_case(monkeypatch):
 	assert torch.equal(z, y)
 	p = x.clone().requires_grad_()
 	assert not layer(p).requires_grad
+
+
+def test_workspace_outlives_the_call(monkeypatch):
+	"""The library runs without the GIL, so another thread may replace the workspace meanwhile: the call keeps the one it was given.  A callback
+	stands for the library here and launches nothing."""
+	import ctypes
+	import gc
+	layer = _layer(256, 128, 128)
+	x = torch.randn(2, 256, device='cuda').half()
+	layer(x)
+	l, host = _lib.lib(), _lib.host()
+	names = ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes', 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')
+	addresses = [ctypes.cast(getattr(l, n), ctypes.c_void_p).value for n in names]
+	table = {(0, torch.cuda.current_stream().cuda_stream): torch.zeros(64 << 20, dtype=torch.uint8, device='cuda')}
+	freed = []
+
+	def replaced(*a):
+		gc.collect()
+		before = torch.cuda.memory_allocated()
+		table.clear()
+		freed.append(before - torch.cuda.memory_allocated())
+		return 0
+	callback = ctypes.CFUNCTYPE(ctypes.c_int, *_lib._SIGNATURES['gptq_qmatmul'][1])(replaced)
+	monkeypatch.setattr(_lib, '_workspaces', table)
+	try:
+		host.bind(*(ctypes.cast(callback, ctypes.c_void_p).value if n == 'gptq_qmatmul' else a for n, a in zip(names, addresses)))
+		assert layer(x) is not None
+	finally:
+		host.bind(*addresses)
+	assert freed == [0] and not table
