@@ -332,6 +332,13 @@ static int launch_narrow(const CUtensorMap &tm0, const CUtensorMap &tm1, const S
 	}
 }
 
+// A call that hands x on through the workspace (gathered or normalised by a kernel of its own) is two launches.  Another thread that calls with
+// the same workspace on the same stream must not get in between: its x would be multiplied.  Held for the two launches, not for their execution.
+static std::mutex &workspace_lock(const void *workspace) {
+	static std::mutex locks[64];
+	return locks[(reinterpret_cast<uintptr_t>(workspace) >> 9) & 63];
+}
+
 template <int NSTREAM, int EPI>
 static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1, void *workspace, size_t ws_bytes,
 						 cudaStream_t stream, size_t gather_off = (size_t)-1) {
@@ -351,6 +358,8 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 	const size_t dec_need = (p.perm || p.rms_w) ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
 	const bool dec = gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow &&
 					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM, EPI == EPI_ROPE)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
+	std::unique_lock<std::mutex> together;
+	if (p.perm || (dec && p.rms_w)) together = std::unique_lock<std::mutex>(workspace_lock(workspace));
 	if (p.perm) {
 		// act-order: x[:, perm] once, into the workspace behind the chosen kernel's scratch (or at the offset the caller planned)
 		const size_t off = (gather_off != (size_t)-1) ? gather_off : gather_offset(dec ? dec_ws_bytes(p.M) : words_offset(need) + words_bytes(p.M, need));

@@ -50,12 +50,13 @@ int gptq_last_cuda_error(void);
 /*
  * Bytes of scratch that gptq_qmatmul / gptq_gateup_silu / gptq_qkv_rope need for a
  * problem of this size (split-K partial sums, per-tile arrival counters, and for act-order
- * decode calls the gathered copy of x).  The
+ * decode calls the gathered, for a folded RMSNorm the normalised copy of x).  The
  * caller allocates it once per stream, ZEROES it once, and hands it to every call;
  * the kernels leave the counter area (the first 16 KiB, status word in its last 4 bytes) zeroed again, except
  * after a non-zero status: a launch that gave up leaves counters and hand-over flags behind, so wait for the
  * stream and zero the first 16 KiB before the next call.  Two calls that overlap on the
- * GPU must not share one workspace.  Replaces the `torch.empty` + 1-D launch grid
+ * GPU must not share one workspace; several host threads may use one on one stream (the launches of
+ * a call that passes x through the workspace are kept together).  Replaces the `torch.empty` + 1-D launch grid
  * set-up of the reference wrapper (quant_linear.py:259-263).
  */
 size_t gptq_workspace_bytes(int M, int K, int N);
@@ -249,8 +250,9 @@ int gptq_attn_prompt(const void *q, int64_t q_sb, int64_t q_st, int64_t q_sh, co
  * RMSNorm folded into the decode kernels (M <= 16).  No counterpart in the reference, whose
  * decoder layer runs the HF LlamaRMSNorm module between its fused ops.  A decode step otherwise
  * spends two extra launches per layer on the norm; here the projection that produces the
- * hidden state also leaves per-tile sums of squares, and the next fused op scales x while it
- * stages it:
+ * hidden state also leaves per-tile sums of squares, and the next fused op scales x: while it
+ * stages it, or (the tensor-memory kernel) in a kernel of its own that leaves the normalised rows
+ * in the workspace:
  *   gptq_qmatmul_sumsq   = gptq_qmatmul, and sumsq_out[row * (N/32) + c] = sum over columns
  *                          32c .. 32c+31 of y^2 (y as rounded to fp16).  N % 128 == 0.
  *   gptq_gateup_silu_rms = gptq_gateup_silu on x * rsqrt(sum_t sumsq_in[row*sumsq_tiles + t] / K

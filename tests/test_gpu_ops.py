@@ -989,3 +989,43 @@ def test_rotary_outputs_that_do_not_start_on_8_bytes(G, b, t):
 	for got, ref in ((k, want[1]), (v, want[2])):
 		assert torch.equal(got[..., :D].transpose(1, 2), ref) and bool((got[..., D:] == 7.0).all())
 	assert bool((q[:, H * D:] == 7.0).all()) and _lib.kernel_status() == 0
+
+
+@pytest.mark.parametrize('act', [False, True])
+def test_two_threads_on_one_stream(G, act):
+	"""Calls that hand x on through the workspace (a folded norm ahead of the tensor-memory kernel, the gather of an act-order layer), from
+	two threads on one stream: every result has the bits that the same call gives alone."""
+	import sys
+	import threading
+	from gptq_triton_b200 import _lib
+	M, K, N, gs, calls = 16, 4096, 256, 128, 4000
+	t, u = ([d[n].cuda() for n in ('qweight', 'qzeros', 'scales')] for d in (synth(K, N, gs, 1), synth(K, N, gs, 2)))
+	perm = torch.randperm(K, generator=torch.Generator().manual_seed(1)).int().cuda()
+	norm_w = torch.ones(K, dtype=torch.float16, device='cuda')
+	xs = [acts((M, K), seed=s).cuda() * (s + 1) for s in range(2)]
+	sums = [x.float().pow(2).view(M, K // 32, 32).sum(-1).contiguous() for x in xs]
+	outs = torch.empty((2, calls + 1, M, N), dtype=torch.float16, device='cuda')
+	ws, P, st, l = _lib.workspace(xs[0].device, M, K, N), _lib.ptr, _lib.stream_ptr(xs[0].device), _lib.lib()
+	size, f = ws.numel(), l.gptq_qmatmul if act else l.gptq_gateup_silu_rms
+	if act:
+		args = [lambda y, i=i: (P(xs[i]), *map(P, t), None, P(perm), None, None, N, y, M, K, N, gs, K, N, P(ws), size, st) for i in range(2)]
+	else:
+		args = [lambda y, i=i: (P(xs[i]), *map(P, t), *map(P, u), None, None, y, M, K, N, gs, K, N, P(ws), size, st, P(norm_w), P(sums[i]), K // 32, 1e-6) for i in range(2)]
+	made = [[args[i](outs[i].data_ptr() + j * M * N * 2) for j in range(calls + 1)] for i in range(2)]
+	assert f(*made[0][calls]) == 0 and f(*made[1][calls]) == 0          # alone
+	start, codes = threading.Barrier(2), [set(), set()]
+
+	def work(i):
+		start.wait()
+		for a in made[i][:calls]:
+			codes[i].add(f(*a))
+	interval = sys.getswitchinterval()
+	try:
+		sys.setswitchinterval(1e-6)
+		threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+		[th.start() for th in threads]
+		[th.join() for th in threads]
+	finally:
+		sys.setswitchinterval(interval)
+	torch.cuda.synchronize()
+	assert codes == [{0}, {0}] and int((outs[:, :calls] != outs[:, calls:]).flatten(2).any(-1).sum()) == 0
