@@ -242,6 +242,10 @@ __global__ void __launch_bounds__(DN_THREADS, 2) dense_skinny_kernel(const Dense
 constexpr int RG_ROWS = 5, RG_STAGES = 5, RG_BOX = 2048, RG_MIN_SMEM = 120 * 1024;
 constexpr int RG_STATIC = (2 * DN_WARPS * SK_M * SK_REDLD + RP_SMEM) * (int)sizeof(float) + DN_WARPS * RG_STAGES * 8 + 64 + 1024;
 
+// One verdict for the whole warp, which goes on to MMAs and shares the stage.
+__device__ __noinline__ bool rg_wait_slow(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)); }
+__device__ __forceinline__ bool rg_wait(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || rg_wait_slow(bar, parity); }
+
 __global__ void __launch_bounds__(DN_THREADS, 1) dense_ring_kernel(const __grid_constant__ CUtensorMap tmw, const __grid_constant__ DenseArgs p, int stages) {
 	extern __shared__ __align__(1024) unsigned char rg_smem[];
 	__shared__ float s_red[2][DN_WARPS][SK_M][SK_REDLD];
@@ -311,7 +315,10 @@ __global__ void __launch_bounds__(DN_THREADS, 1) dense_ring_kernel(const __grid_
 		float d[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
 		for (int u = 0; u < count; ++u) {
-			ok = ok && mbar_wait_bounded(bars + 8 * cs, parity);
+			if (ok && !rg_wait(bars + 8 * cs, parity)) {
+				ok = false;
+				left = 0;                                // no further copies; the sums are worthless, the status says so
+			}
 			uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
 			if (live) {
 				x0 = *reinterpret_cast<const uint4 *>(xrow + u * 128);

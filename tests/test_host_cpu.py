@@ -181,6 +181,18 @@ def test_projections_that_store_many_cache_rows_do_not_start_their_successor_ear
 			assert text.index('pdl_wait();') < text.index('pdl_trigger();')
 
 
+def test_dense_ring_kernel_gives_up_as_a_whole_warp():
+	"""A wait that runs out has to be known to every lane: the MMAs behind it are the warp's, and lane 0 reports.  By the source."""
+	from gptq_triton_b200.build import CSRC
+	text = (CSRC / 'dense' / 'dense_skinny.cu').read_text()
+	waits = [line for line in text.splitlines() if 'mbar_wait_bounded(' in line or 'mbar_try_wait(' in line]
+	assert waits and all('__all_sync(0xffffffffu, mbar_' in line for line in waits)
+	kernel = text[text.index('dense_ring_kernel('):]
+	kernel = kernel[:kernel.index('\n}\n')]
+	given_up = kernel[kernel.index('!rg_wait('):]
+	assert given_up.index('left = 0;') < given_up.index('load();') < given_up.index('if (!ok)') < given_up.index('atomicExch(p.status')
+
+
 def test_clear_kernel_status_clears_the_whole_control_area(monkeypatch):
 	"""Arrival counters and hand-over flags of a launch that gave up go with its status, in retired workspaces too (a captured graph may
 	still use one); what lies behind the first 16 KB stays."""
