@@ -160,8 +160,8 @@ struct RowWeights {
 		for (int i = 0; i < RP_REGS; ++i) {
 			const int u = threadIdx.x + i * DN_THREADS;
 			if (u < (p.ld >> 2)) {
-				gain[i] = rp_gain(p.gain, u);
-				shift[i] = rp_shift(p.shift, u);
+				gain[i] = rp_gain(p.y ? p.gain : nullptr, u);          // (gain and shift belong to y: without it they are not read)
+				shift[i] = rp_shift(p.y ? p.shift : nullptr, u);
 				w[i] = rp_gain(p.fin_w, u);
 				b[i] = rp_shift(p.fin_b, u);
 			}

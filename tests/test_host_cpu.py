@@ -193,6 +193,16 @@ def test_dense_ring_kernel_gives_up_as_a_whole_warp():
 	assert given_up.index('left = 0;') < given_up.index('load();') < given_up.index('if (!ok)') < given_up.index('atomicExch(p.status')
 
 
+def test_gain_and_shift_are_read_with_y_only():
+	"""Rows without a y have no gain or shift; whatever the two pointers hold then is not to be read ahead of the wait either.  By the source."""
+	from gptq_triton_b200.build import CSRC
+	text = (CSRC / 'dense' / 'dense.cuh').read_text()
+	weights = text[text.index('struct RowWeights'):]
+	weights = weights[:weights.index('\n};')]
+	reads = [line for line in weights.splitlines() if 'p.gain' in line or 'p.shift' in line]
+	assert len(reads) == 2 and all('p.y ? p.' in line for line in reads)
+
+
 def test_clear_kernel_status_clears_the_whole_control_area(monkeypatch):
 	"""Arrival counters and hand-over flags of a launch that gave up go with its status, in retired workspaces too (a captured graph may
 	still use one); what lies behind the first 16 KB stays."""
