@@ -378,6 +378,21 @@ int ring_stages(const DenseArgs &a) {
 	return n >= 3 ? n : 0;
 }
 
+// Where the kernel with two CTAs per SM is the faster one all the same (us, that one / ring; `smem`: what its rows take).
+//   Two K slices per warp on many tiles: the barrier and the sums of a tile outweigh its copies.  768 -> 32000 12.9 / 13.9, -> 64000 22.9 / 26.3, 576 -> 64000
+//   20.8 / 25.3; on fewer tiles the other way round (768 -> 4768 4.4 / 3.8, 5 rows -> 8192 6.1 / 5.7, rows prepared here -> 16384 14.0 / 13.3); with a whole
+//   multiple of slices 1024 -> 32000 14.9 / 14.6, -> 64000 26.6 / 28.2.  One slice
+//   per warp (512 -> 64000 .91) and three (1280 .92) are not affected, four uneven ones (1664 -> 64000 43.0 / 44.0) a little.
+//   Long rows, where a tile takes as long as the launch, and tiles that fill as many rounds here as half rounds there: 8192 -> 7136 25.1 / 27.1, -> 2400 12.8 / 13.3,
+//   -> 12240 37.4 / 38.9; with one round less the ring wins (-> 4768 .88, -> 9504 .96), and so it does where the rows leave room for one CTA only or for
+//   little L1 beside two (5 rows .75).
+bool ring_loses(const DenseArgs &a, int ntiles, size_t smem) {
+	const int units = (a.K + 63) >> 6, sms = dn_sm_count();
+	if (units > 8 && units <= 16) return ntiles > (units == 16 ? 2048 : a.prep ? 1280 : 640);
+	if (units > 24 && units < 32) return ntiles > 1536;
+	return a.K >= 8192 && smem <= 68 * 1024 && !(a.prep && ntiles <= 2 * sms) && (ntiles + sms - 1) / sms == 2 * ((ntiles + 2 * sms - 1) / (2 * sms));
+}
+
 int launch_ring(const DenseArgs &a, int stages, cudaStream_t stream) {
 	alignas(64) CUtensorMap tmw;
 	if (int rc = dense_tensor_map(a.w, a.N, a.K, a.ldw, 16, 64, &tmw)) return rc;
@@ -398,7 +413,7 @@ int launch(const DenseArgs &a, cudaStream_t stream) {
 	// Up to five rows: per decode step of a latent-attention model in us, this kernel / the one below: 8 layers of 2048 hidden, 1 row 381 / 433; 4 and
 	// 3 layers of 2048 and 4096, 2 rows 228 / 251 and 358 / 361, 5 rows 279 / 294 and 397 / 421; 8 rows 297 / 341 and 486 / 472 (there the rows
 	// of the widest layers do not fit, and every change between the two kernels' shared-memory splits costs more than the kernel gains).
-	if (sizeof(T) == 2 && a.M <= RG_ROWS)
+	if (sizeof(T) == 2 && a.M <= RG_ROWS && !ring_loses(a, ntiles, smem))
 		if (const int stages = ring_stages(a)) return launch_ring(a, stages, stream);
 	const int waves = (ntiles + slots - 1) / slots;
 	return dn_launch(dense_skinny_kernel<T, false>, dim3((ntiles + waves - 1) / waves), dim3(DN_THREADS), smem, stream, a, 1);

@@ -78,6 +78,18 @@ def test_projection_of_few_rows(control, M, K, N):
 	assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
 
 
+@pytest.mark.parametrize('M', [1, 4])
+@pytest.mark.parametrize('K,N', [(576, 10240), (576, 10256), (1024, 32768), (1024, 32784), (1664, 24576), (1664, 24592), (8192, 2352), (8192, 2400), (8192, 4768), (8192, 7136)])
+def test_projection_beside_the_lines_between_the_kernels(control, M, K, N):
+	"""Sizes on both sides of each line up to which few rows stream through shared memory."""
+	from gptq_triton_b200 import dense
+	gen = torch.Generator(device='cuda').manual_seed(K + N)
+	x, w = torch.randn((M, K), generator=gen, device='cuda').to(B16), torch.randn((N, K), generator=gen, device='cuda').to(B16)
+	got = dense.linear(x, w, control)
+	ref, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+	assert ((got[:, :N] - ref).abs() <= 2.0 ** -24 * K * size).all()
+
+
 @pytest.mark.parametrize('dtype', [F32, B16])
 @pytest.mark.parametrize('M', [1, 2, 3, 8, 40, 200])
 def test_mlp_sublayer(control, dtype, M):
