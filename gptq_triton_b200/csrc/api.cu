@@ -416,6 +416,20 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 			  : launch_skinny_inst<4, NSTREAM, false, 0, EPI>(tm0, tm1, p, grid, smem, stream);
 }
 
+template <int STAGES>
+static int launch_attn_decode(const AttnParams &p, int batch, cudaStream_t stream) {
+	constexpr size_t smem = (size_t)STAGES * AT_STAGE_BYTES + 64;
+	static bool ready[64] = {false};
+	int dev = 0;
+	if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GPTQ_ERR_CUDA;
+	if (!ready[dev]) {
+		cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+		if (e != cudaSuccess) return cuda_status(e);
+		ready[dev] = true;
+	}
+	return launch_ex(attn_decode_kernel<STAGES>, dim3(p.splits, p.heads, batch), dim3(AT_THREADS, 1, 1), smem, stream, p);
+}
+
 // Folded RMSNorm (consumer side): decode kernel only, x read in order, at most 256 partial sums per row.
 static int check_rms(const void *rms_weight, const float *sumsq_in, int sumsq_tiles, float eps, int M, const int32_t *g_idx,
 					 const int32_t *perm) {
@@ -614,22 +628,15 @@ int gptq_attn_decode(const void *q, int64_t q_stride_b, const void *kcache, cons
 	p.kv_stride_b = kv_stride_b; p.kv_stride_h = kv_stride_h;
 	p.pos = pos; p.out = (__half *)out; p.out_stride_b = out_stride_b;
 	p.scale = scale; p.heads = heads; p.splits = splits;
-	// More (sequence, head) pairs than fit at two CTAs per SM: two stages, so that three do and their latencies overlap.  Step of 16 sequences of 100 positions, 64 heads,
-	// 8 layers 1461 -> 1377 us; 12 sequences of 900 positions, 32 heads, 4 layers 469 -> 432.  In a single wave three stages are the better ones (8 sequences of 97: 298 / 302).
-	p.stages = batch * heads > 2 * sm_count() ? 2 : AT_STAGES;
 	p.ws_ticket = reinterpret_cast<int *>(workspace);
 	p.ws_partial = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(workspace) + AT_TICKET_BYTES);
-	{
-		static bool ready[64] = {false};
-		int dev = 0;
-		if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return GPTQ_ERR_CUDA;
-		if (!ready[dev]) {
-			cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
-			if (e != cudaSuccess) return cuda_status(e);
-			ready[dev] = true;
-		}
-	}
-	return launch_ex(attn_decode_kernel, dim3(splits, heads, batch), dim3(AT_THREADS, 1, 1), (size_t)p.stages * AT_STAGE_BYTES + 64, reinterpret_cast<cudaStream_t>(stream), p);
+	// Two stages, so that three CTAs fit an SM, where that saves more of the waves than each of them gets longer (three CTAs share what two had), or any where the
+	// cache is short and a CTA's latency is most of its time.  Two stages / three, us: 384 pairs (one wave / two), 100 positions .70, 4000 .75; 640 (two / three) .79,
+	// .93; 1024 (three / four), 100 .86, 900 1.00, 4000 1.05; 512 (two either way), 100 1.01, 500 33.8 / 30.7, 2000 104.5 / 86.5.  In a single wave three stages are
+	// the better ones.  Step of 16 sequences of 100 positions, 64 heads, 8 layers 1461 -> 1377 us.
+	const int pairs = batch * heads, sms = sm_count(), waves2 = (pairs + 2 * sms - 1) / (2 * sms), waves3 = (pairs + 3 * sms - 1) / (3 * sms);
+	const bool two = 3 * waves3 <= 2 * waves2 || (waves3 < waves2 && len_hint <= 1024);
+	return two ? launch_attn_decode<2>(p, batch, reinterpret_cast<cudaStream_t>(stream)) : launch_attn_decode<AT_STAGES>(p, batch, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // Shared-memory layout of qkv_attn_kernel for nc chunks of 128 K-rows per CTA; returns the total.

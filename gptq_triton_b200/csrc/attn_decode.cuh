@@ -26,7 +26,6 @@ constexpr int AT_STATUS_SLOT = AT_TICKET_BYTES / 4 - 1;      // same word as the
 constexpr int AT_CHUNK = 64;           // keys per stage
 constexpr int AT_STAGES = 3;
 constexpr int AT_STAGE_BYTES = 2 * AT_CHUNK * AT_D * 2;      // K rows then V rows: 32 KB
-constexpr int AT_SMEM_BYTES = AT_STAGES * AT_STAGE_BYTES + 64;
 constexpr int AT_FRESH = 16;           // newest positions that are never read ahead of the dependency wait
 
 struct AttnParams {
@@ -39,7 +38,6 @@ struct AttnParams {
 	long long out_stride_b;
 	float scale;
 	int heads, splits;
-	int stages;               // 2 or AT_STAGES
 	float *ws_partial;        // [b*heads][splits][130]
 	int *ws_ticket;           // [b*heads]
 };
@@ -50,7 +48,8 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void *src, uint
 				 : "memory");
 }
 
-__global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(const AttnParams p) {
+template <int STAGES>                  // AT_STAGES, or two where three CTAs per SM save a wave (gptq_attn_decode)
+__global__ void __launch_bounds__(AT_THREADS, STAGES == AT_STAGES ? 2 : 3) attn_decode_kernel(const AttnParams p) {
 	extern __shared__ __align__(128) unsigned char at_smem[];
 	const int split = blockIdx.x, head = blockIdx.y, b = blockIdx.z;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -68,7 +67,7 @@ __global__ void __launch_bounds__(AT_THREADS, 3) attn_decode_kernel(const AttnPa
 	__shared__ float s_m[AT_GROUPS], s_l[AT_GROUPS];
 	float(*s_acc)[AT_D] = reinterpret_cast<float(*)[AT_D]>(at_smem);      // [AT_GROUPS][128], over the drained stages
 	__shared__ int s_last;
-	const int nst = p.stages;
+	constexpr int nst = STAGES;
 	const uint32_t bar0 = smem_u32(at_smem + nst * AT_STAGE_BYTES);
 	if (tid == 0) {
 		for (int s = 0; s < nst; ++s) mbar_init(bar0 + 8 * s, 1);

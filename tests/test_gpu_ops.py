@@ -417,6 +417,27 @@ def test_attn_decode_of_more_pairs_than_a_wave(G, heads):
 	assert _lib.kernel_status() == 0
 
 
+@pytest.mark.parametrize('heads', [55, 56, 74, 75, 128])
+def test_attn_decode_beside_the_lines_between_two_and_three_stages(G, heads):
+	"""Eight sequences: 440 | 448 pairs (one wave of three CTAs per SM | two), 592 | 600 (two waves of two | three), 1024 (two stages up to 1024 positions only, by
+	the hint): the number of stages changes no bit."""
+	from gptq_triton_b200 import _lib
+	from gptq_triton_b200.fused_attention import attn_decode
+	b, S, D = 8, 320, 128
+	positions = torch.tensor([0, 63, 64, 127, 128, 200, 256, 319], dtype=torch.int32)
+	gen = torch.Generator(device='cuda').manual_seed(heads)
+	q, kc, vc = (torch.randn(shape, generator=gen, device='cuda').half() for shape in ((b, 1, heads, D), (b, heads, S, D), (b, heads, S, D)))
+	outs = [attn_decode(q.transpose(1, 2), kc, vc, positions.view(b, 1).cuda(), len_hint=hint) for hint in (S, 1025)]
+	few = torch.cat([attn_decode(q[:, :, h:h + 32].contiguous().transpose(1, 2), kc[:, h:h + 32].contiguous(), vc[:, h:h + 32].contiguous(), positions.view(b, 1).cuda(), len_hint=64)
+					 for h in range(0, heads, 32)], -1)          # at most 256 pairs: three stages, keys not split
+	s = torch.einsum('bhd,bhsd->bhs', q[:, 0].double(), kc.double()) / D ** 0.5
+	s.masked_fill_(torch.arange(S, device='cuda')[None, None] > positions.cuda()[:, None, None], -float('inf'))
+	ref = torch.einsum('bhs,bhsd->bhd', torch.softmax(s, -1), vc.double()).reshape(b, -1)
+	for out in outs:
+		assert torch.equal(out, few) and O.max_rel_err(out.view(b, -1).cpu(), ref.float().cpu()) <= TOL
+	assert _lib.kernel_status() == 0
+
+
 @pytest.mark.parametrize('M,K', [(1, 4096), (5, 512), (16, 11008)])
 def test_rmsnorm_kernel(G, M, K):
 	from gptq_triton_b200.fused_attention import rmsnorm
