@@ -254,18 +254,36 @@ static void plan_skinny(SkinnyParams &p, int nstream, int &kw, dim3 &grid, size_
 //   3072 -> 2 x 8192              M = 2  12.4 / 10.9   M = 3  12.5 / 12.4   M = 4   12.4 / 13.5   M = 16  12.9 / 24.8
 //   4096 -> 2 x 11008             M = 2  17.2 / 15.9   M = 3  17.2 / 17.3   M = 4   17.2 / 18.3   M = 16  17.8 / 35.2
 //   8192 -> 2 x 22016, norm       M = 1  50.1 / 49.8   M = 2  51.5 / 54.3   M = 16  53.9 / 119
+//   11008 -> 2 x 11008            M = 2  37.4 / 36.4   M = 3   .97 of it (22016 -> 2 x 5504 the same)
+// Exceptions among them: few tiles of a deep K, as below, and wide layers of a short K, whose units do not divide among the CTAs:
+//   8192 -> 2 x 256, norm         M = 3  14.5 / 9.7    M = 6  14.9 / 12.4  M = 8   1.07 of it
+//   4096 -> 2 x 512, norm         M = 3   9.4 / 7.8    M = 4   9.6 / 8.3   M = 5   .97 of it
+//   1024 -> 2 x 5504              M = 3   8.2 / 6.8    M = 4   8.0 / 7.1   M = 5   .99 of it
+// x of an act-order layer is gathered ahead, by CTAs that run on the free SMs while the kernel in front is busy: with more than some 30 of them (11 per row at
+// K = 22016) the gather takes longer than the weights wait for it.  22016 -> 4096, perm  M = 4  26.4 / 21.3   M = 5  27.9 / 24.0
+// At 3 rows 1536 -> 2 x 2816, 2048 -> 2 x 2048 and 3072 -> 2 x 2816 are within 0.2 us of each other (1.02 to 1.04), layers beside them gain 5 to 20 %.
+// The same at both ends of the single layers:
+//   512 -> 24576                  M = 5   6.7 / 5.8    M = 6   6.7 / 6.0
+//   5504 -> 12288 (34 MB)         M = 4  13.5 / 13.1   M = 5   .93 of it
+//   11008 -> 12288 (68 MB)        M = 3  22.2 / 20.8   M = 4   .75 of it
 // A narrow layer with a deep K is the exception: every tile of 128 columns is spread over many CTAs, and the last one adds their sums.
 //   4096 -> 2048 (16 tiles)       M = 5   6.5 / 6.3    M = 7   6.5 / 6.8    M = 16  7.6 / 8.8
 //   8192 -> 2048                  M = 4   7.5 / 5.8    M = 5   7.5 / 7.5    M = 16  8.6 / 10.5
 //   8192 -> 1024 (8 tiles)        M = 7   8.6 / 8.4    M = 9   8.8 / 9.2    M = 16 10.2 / 9.7
 // The lines of the layers of fewer than 48 tiles are those of an earlier form of the kernel, which took 1 us more; they are pinned by tests.
-static int dec_min_rows(int K, int N, int nstream, bool rope) {
+static int dec_min_rows(int K, int N, int nstream, bool rope, bool gathered) {
 	const int tiles = N / 128;
 	if (nstream == 1 && tiles < 30 && (rope ? K >= 1536 : K > 2048)) return tiles <= 16 ? 17 : 9;
 	const double mb = (double)K * N * nstream / 2e6;
+	if (gathered && K > 12288) return mb >= 64 ? 4 : mb >= 20 ? 6 : 7;
+	if (nstream == 2) {
+		if (N >= 256 && N <= 768 && K >= 3072 && mb < 4.2) return N == 256 && K >= 8192 ? 7 : 5;
+		if (K <= 512 ? N > 16384 : K <= 1024 && N > 4096 && N < 8192) return 5;
+		return mb >= 100 && K <= 8192 ? 2 : 3;
+	}
 	if (mb >= 100) return 2;
-	if (nstream == 2 || mb >= 64) return 3;
-	return mb >= 32 ? 4 : mb >= 24 || tiles >= 48 ? 5 : mb >= 20 ? 6 : 7;
+	if (mb >= (N > 16384 ? 64 : 80)) return 3;
+	return mb >= 32 ? 4 : mb >= 24 || (tiles >= 48 && (K > 512 || tiles < 80)) ? 5 : mb >= 20 ? 6 : 7;
 }
 
 // Narrow geometry (one 32-column strip and the whole of K per CTA, no split-K): worth it when
@@ -357,7 +375,7 @@ static int launch_skinny(SkinnyParams &p, const int32_t *qw0, const int32_t *qw1
 	// the tensor-memory kernel, where it is the faster one and the workspace has room for its scratch (and the gathered or normalised x behind that)
 	const size_t dec_need = (p.perm || p.rms_w) ? gather_offset(dec_ws_bytes(p.M)) + gather_bytes(p.M, p.K) : dec_ws_bytes(p.M);
 	const bool dec = gather_off == (size_t)-1 && p.ar_world <= 1 && g_force_splitk == 0 && !narrow &&
-					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM, EPI == EPI_ROPE)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
+					 p.M >= (g_dec_min_rows ? g_dec_min_rows : dec_min_rows(p.K, p.N, NSTREAM, EPI == EPI_ROPE, p.perm != nullptr)) && dec_shape_ok(p.M, p.K, p.N, p.groupsize) && ws_bytes >= dec_need;
 	std::unique_lock<std::mutex> together;
 	if (p.perm || (dec && p.rms_w)) together = std::unique_lock<std::mutex>(workspace_lock(workspace));
 	if (p.perm) {

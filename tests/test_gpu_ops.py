@@ -929,6 +929,28 @@ def test_which_decode_kernel_runs_for_wide_and_paired_layers(G, pair, K, N, M, t
 	assert ((outs[1].float() - outs[2].float()).abs().max() / outs[2].float().abs().max()).item() <= 2 * TOL
 
 
+@pytest.mark.parametrize('kind,K,N,M,tensor_memory', [
+	('pair', 4096, 512, 4, False), ('pair', 4096, 512, 5, True), ('pair', 8192, 256, 6, False), ('pair', 8192, 256, 7, True), ('pair', 5632, 768, 3, True), ('pair', 1024, 5504, 4, False),
+	('pair', 1024, 5504, 5, True), ('pair', 512, 16512, 4, False), ('pair', 512, 16384, 3, True), ('pair', 8320, 12160, 2, False), ('plain', 512, 10240, 6, False), ('plain', 512, 10112, 5, True),
+	('plain', 9600, 16384, 3, False), ('plain', 9600, 16512, 3, True), ('perm', 12416, 1408, 4, False), ('perm', 12288, 4096, 5, True), ('perm', 12416, 4096, 5, False)])
+def test_which_decode_kernel_runs_at_the_exceptions(G, kind, K, N, M, tensor_memory):
+	"""The same for the exceptions among the paired, the wide and the act-order layers."""
+	from gptq_triton_b200 import _lib
+	layers = [[v.cuda() for v in (t['qweight'], t['scales'], t['qzeros'])] for t in (synth(K, N, 128, seed) for seed in range(1 + (kind == 'pair')))]
+	x = acts((1, M, K), seed=M).cuda()
+	perm = torch.randperm(K, generator=torch.Generator().manual_seed(1)).int().cuda() if kind == 'perm' else None
+	outs = []
+	try:
+		for rows in (0, 1, 17):
+			_lib.lib().gptq_debug_dec_min_rows(rows)
+			outs.append(G.gateup_silu(128, x, *layers[0], *layers[1]) if kind == 'pair' else G.qmatmul(128, x, *layers[0], perm=perm))
+	finally:
+		_lib.lib().gptq_debug_dec_min_rows(0)
+	assert not torch.equal(outs[1], outs[2])
+	assert torch.equal(outs[0], outs[1] if tensor_memory else outs[2])
+	assert ((outs[1].float() - outs[2].float()).abs().max() / outs[2].float().abs().max()).item() <= 2 * TOL
+
+
 @pytest.mark.parametrize('M', [17, 40, 144, 145])
 @pytest.mark.parametrize('K,gs', [(192, 64), (448, 64), (192, 192)])
 def test_prefill_of_large_scales_behind_an_odd_number_of_k_blocks(G, M, K, gs):
