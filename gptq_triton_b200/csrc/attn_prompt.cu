@@ -302,7 +302,7 @@ int gptq_attn_prompt_prepare(const void *mask, int64_t mask_sb, int64_t mask_st,
 int gptq_attn_prompt(const void *q, int64_t q_sb, int64_t q_st, int64_t q_sh, const void *k, const void *v, const void *mask, int64_t mask_sb, int64_t mask_st, int mask_b, int b,
 					 int heads, int t, int S, float scale, void *out, const void *scratch, size_t scratch_bytes, gptq_stream_t stream) {
 	if (int rc = prompt_shape(mask, mask_sb, mask_st, mask_b, b, heads, t, S, scratch, scratch_bytes)) return rc;
-	if (!q || !k || !v || !out) return GPTQ_ERR_INVALID;
+	if (!q || !k || !v || !out || !(scale > 0.f && scale <= 3.402823466e38f)) return GPTQ_ERR_INVALID;
 	if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || ((q_sb | q_st | q_sh) & 7)) return GPTQ_ERR_ALIGN;
 	PromptParams p = {};
 	p.q = (const __half *)q; p.k = (const __half *)k; p.v = (const __half *)v; p.mask = (const __half *)mask;

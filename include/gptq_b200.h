@@ -235,7 +235,7 @@ int gptq_embed_rmsnorm(const void *table, int64_t ldt, int64_t n_rows, const int
  * matmul / softmax / matmul, fused_attention.py:105-146).  mask: element strides mask_sb, mask_st, 1 of [mask_b, t, S], mask_b = b or 1 (shared).
  *   gptq_attn_prompt_prepare   classifies the tiles of the mask into `scratch` and copies the `past` cached rows (element strides per sequence
  *                              and head, rows of 128) to the front of k, v [b, heads, S, 128]
- *   gptq_attn_prompt           out [b, t, heads * 128] = softmax(q k^T scale + mask) v; a query that sees nothing gets zeros.  scratch NULL:
+ *   gptq_attn_prompt           out [b, t, heads * 128] = softmax(q k^T scale + mask) v, scale > 0; a query that sees nothing gets zeros.  scratch NULL:
  *                              no tile of the mask has been classified
  */
 size_t gptq_attn_prompt_scratch_bytes(int b, int t, int S);

@@ -115,3 +115,10 @@ def test_python_ops_refuse_cpu_tensors():
 		g.triton_matmul4(128, x, qw, sc, qz)
 	with pytest.raises(AssertionError):
 		g.triton_matmul4(128, torch.zeros(1, 250, dtype=torch.float16), qw, sc, qz)
+
+
+@pytest.mark.parametrize('scale', [0.0, -0.5, float('nan'), float('inf')])
+def test_prompt_attention_refuses_a_scale_that_is_not_positive(lib, scale):
+	"""Open tiles are scaled behind their maximum and hidden columns are minus infinity times the scale, so anything but a positive finite number is an error."""
+	fake = ctypes.c_void_p(0x1000)
+	assert lib.gptq_attn_prompt(fake, 128, 128, 128, fake, fake, fake, 64, 64, 1, 1, 1, 8, 64, scale, fake, None, 0, None) == -1
