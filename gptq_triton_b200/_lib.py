@@ -1,13 +1,15 @@
 """ctypes binding of libgptq_b200.so (declared in include/gptq_b200.h).
 
 There is no fallback: if the library is missing or a kernel cannot run, an exception is
-raised.  The library is built in-tree by `python -m gptq_triton_b200.build`.
+raised.  The library is built in-tree by `python -m gptq_triton_b200.build`.  (The extension
+module of host() is another way into the same library, and can be missing.)
 """
 from __future__ import annotations
 
 import ctypes
 import functools
 import os
+import warnings
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p
 from pathlib import Path
 from typing import Dict, Optional, Tuple
@@ -18,7 +20,7 @@ _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / 'libgptq_b200.so'
 
 _lib: Optional[ctypes.CDLL] = None
-_host = None          # extension module csrc/host/calls.cpp, bound to the library
+_host = None          # extension module csrc/host/calls.cpp, bound to the library, or what stands for it (see host())
 
 _P = c_void_p
 _SIGNATURES = {
@@ -117,21 +119,37 @@ def lib() -> ctypes.CDLL:
 			l.gptq_debug_max_stages(int(os.environ['GPTQ_B200_STAGES']))      # ring depth of the decode kernel (A/B measurements)
 		if os.environ.get('GPTQ_B200_PDL', '1') == '0' and hasattr(l, 'gptq_debug_set_pdl'):
 			l.gptq_debug_set_pdl(0)      # opt out of programmatic dependent launch (A/B measurements)
-		try:
-			from . import _host as module
-		except ImportError as e:
-			raise ImportError(f'{_PKG / "_host.so"} is missing or does not fit this torch: build it with `python -m gptq_triton_b200.build`.') from e
-		address = lambda name: ctypes.cast(getattr(l, name), c_void_p).value
-		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes',
-									 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')))
-		_lib, globals()['_host'] = l, module
+		_lib = l
 	return _lib
 
 
+class _Ctypes:
+	"""In the place of the extension module: serves nothing, so every call goes through ctypes."""
+	qmatmul = gateup = qkv = attend = staticmethod(lambda *a: None)
+
+
 def host():
-	"""Layer calls in native code; each returns None when the call is not the plain case, and has then done nothing."""
+	"""Layer calls in native code; each returns None when the call is not the plain case.  Without the module, or with one that was built
+	against another torch, the layers run through ctypes (several microseconds more per call)."""
+	global _host
 	if _host is None:
-		lib()
+		try:
+			l = lib()
+		except ImportError:
+			return _Ctypes          # (said by whatever needs the library)
+		try:
+			from . import _host as module
+			built = getattr(module, 'torch_version', 'unknown')
+			if built != str(torch.__version__):
+				raise ImportError(f'built against torch {built}, this is {torch.__version__}')
+		except ImportError as e:
+			warnings.warn(f'{_PKG / "_host.so"} is not used ({e}): layer calls take several microseconds more; build it with `python -m gptq_triton_b200.build`.', RuntimeWarning)
+			_host = _Ctypes
+			return _host
+		address = lambda name: ctypes.cast(getattr(l, name), c_void_p).value
+		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes',
+									 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')))
+		_host = module
 	return _host
 
 

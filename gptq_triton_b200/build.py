@@ -15,6 +15,7 @@ import subprocess
 import sys
 import sysconfig
 import tempfile
+import warnings
 from pathlib import Path
 from typing import Iterable, Optional
 
@@ -52,7 +53,8 @@ def _host_command(out: str):
 	import torch
 	root = Path(torch.__file__).parent
 	paths = [f'-I{p}' for p in (root / 'include', Path(_nvcc()).resolve().parent.parent / 'include', sysconfig.get_paths()['include'])]
-	return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}', *paths, '-o', out, *map(str, sources('host')),
+	return ['g++', '-O2', '-std=c++17', '-fPIC', '-shared', f'-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}',
+			f'-DGPTQ_TORCH_VERSION="{torch.__version__}"', *paths, '-o', out, *map(str, sources('host')),
 			f'-L{root / "lib"}', '-ltorch_python', '-ltorch_cpu', '-ltorch', '-lc10', '-lc10_cuda']
 
 
@@ -85,11 +87,17 @@ def up_to_date(target: str = 'gptq') -> bool:
 
 
 def build(force: bool = False, verbose: bool = False, only: Optional[Iterable[str]] = None) -> Path:
-	"""Compiles the libraries that are missing or out of date (`only`: names of TARGETS); returns the path of the first."""
+	"""Compiles the libraries that are missing or out of date (`only`: names of TARGETS); returns the path of the first.  The extension module
+	needs g++ and the headers of Python and torch; where it cannot be built the libraries serve every call without it."""
 	targets = list(only) if only else list(TARGETS)
 	for target in targets:
 		if force or not up_to_date(target):
-			_build_one(target, verbose)
+			try:
+				_build_one(target, verbose)
+			except (RuntimeError, OSError) as e:
+				if target != 'host' or only:
+					raise
+				warnings.warn(f'{HOST_LIB.name} was not built: {e}', RuntimeWarning)
 	return TARGETS[targets[0]][0]
 
 

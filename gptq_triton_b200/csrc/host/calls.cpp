@@ -362,4 +362,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }   // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+	PyObject *m = PyModule_Create(&module);
+	if (m && PyModule_AddStringConstant(m, "torch_version", GPTQ_TORCH_VERSION) != 0) Py_CLEAR(m);          // of the torch that it was compiled against
+	return m;
+}

@@ -181,6 +181,58 @@ def test_projections_that_store_many_cache_rows_do_not_start_their_successor_ear
 			assert text.index('pdl_wait();') < text.index('pdl_trigger();')
 
 
+@pytest.mark.parametrize('what', ['missing', 'other torch', 'old'])
+def test_without_the_extension_module_calls_go_through_ctypes(monkeypatch, what):
+	"""The module is another way into the library, not a part of it: missing, or built against another torch, it is left out with one warning."""
+	import sys
+	import types
+	from gptq_triton_b200 import _lib, build
+	build.build()
+	monkeypatch.setattr(_lib, '_host', None)
+	monkeypatch.setattr(_lib, '_lib', None)
+	module = None if what == 'missing' else types.SimpleNamespace(torch_version='1.0', bind=lambda *a: pytest.fail('bound')) if what == 'other torch' else types.SimpleNamespace()
+	monkeypatch.setitem(sys.modules, 'gptq_triton_b200._host', module)
+	if module is not None:
+		monkeypatch.setattr(G, '_host', module, raising=False)
+	else:
+		monkeypatch.delattr(G, '_host', raising=False)
+	assert _lib.lib().gptq_version() >= 100
+	with pytest.warns(RuntimeWarning, match='_host.so is not used'):
+		host = _lib.host()
+	assert all(getattr(host, f)() is None for f in ('qmatmul', 'gateup', 'qkv', 'attend')) and _lib.host() is host
+	with pytest.raises(_lib.GptqB200Error):          # (the error that such a call had before)
+		G.triton_matmul4(128, torch.zeros(1, 256, dtype=torch.float16), torch.zeros(32, 256, dtype=torch.int32), torch.zeros(2, 256, dtype=torch.float16), torch.zeros(2, 32, dtype=torch.int32))
+
+
+def test_cpu_tensors_are_refused_without_the_library(monkeypatch, tmp_path):
+	"""... with the message that says why, which needs no library."""
+	from gptq_triton_b200 import _lib
+	monkeypatch.setattr(_lib, '_host', None)
+	monkeypatch.setattr(_lib, '_lib', None)
+	monkeypatch.setattr(_lib, 'LIB_PATH', tmp_path / 'none.so')
+	with pytest.raises(_lib.GptqB200Error, match='CUDA tensors only'):
+		G.triton_matmul4(128, torch.zeros(1, 256, dtype=torch.float16), torch.zeros(32, 256, dtype=torch.int32), torch.zeros(2, 256, dtype=torch.float16), torch.zeros(2, 32, dtype=torch.int32))
+	with pytest.raises(ImportError):
+		_lib.lib()
+
+
+def test_build_goes_on_without_the_extension_module(monkeypatch):
+	"""g++ or the headers of Python missing: the libraries are built, the module is left out with a warning, unless it was asked for by name."""
+	from gptq_triton_b200 import build
+	built = []
+
+	def one(target, verbose):
+		if target == 'host':
+			raise RuntimeError('g++ failed building _host.so')
+		built.append(target)
+	monkeypatch.setattr(build, '_build_one', one)
+	with pytest.warns(RuntimeWarning, match='_host.so was not built'):
+		assert build.build(force=True) == build.LIB
+	assert built == ['gptq', 'dense']
+	with pytest.raises(RuntimeError):
+		build.build(force=True, only=['host'])
+
+
 def test_dense_ring_kernel_gives_up_as_a_whole_warp():
 	"""A wait that runs out has to be known to every lane: the MMAs behind it are the warp's, and lane 0 reports.  By the source."""
 	from gptq_triton_b200.build import CSRC
