@@ -2,8 +2,9 @@
 //
 // A call of the smallest layer is bound by the host: o_proj of a 7B layer for one token took 16.5 us a call, 5.5 of them on the GPU; the rest was
 // Python (argument checks, torch.empty, nineteen ctypes conversions).  Every function here serves the plain case and returns None for anything
-// else (other types, devices or layouts, tensor subclasses, a missing or small workspace, an active torch-function mode, an error from the library),
-// without having done anything; the caller then goes on in Python, which supports or reports it.
+// else (other types, devices or layouts, tensor subclasses, a missing or small workspace, an active torch-function mode, an error code from the library);
+// the caller then makes the whole call in Python, which supports or reports it.  What has been launched by then (attend() and a gate product come before
+// a code of a later launch) wrote to tensors of its own only.  Exceptions of torch (out of memory, a CUDA error) go to the caller as they are.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -18,6 +19,7 @@
 #include <ATen/ops/silu.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../../include/gptq_b200.h"
@@ -151,16 +153,15 @@ struct Call {
 
 PyObject *none() { Py_RETURN_NONE; }
 
-// Runs f, which returns a new reference or nullptr for "not the plain case"; no C++ exception leaves.
+// Runs f, which returns a new reference or nullptr for "not the plain case"; a C++ exception becomes the Python one that torch makes of it.
 template <typename F>
 PyObject *guarded(F &&f) {
-	try {
-		if (quiet())
-			if (PyObject *r = f()) return r;
-	} catch (...) {
-	}
+	HANDLE_TH_ERRORS
+	if (quiet())
+		if (PyObject *r = f()) return r;
 	PyErr_Clear();
 	return none();
+	END_HANDLE_TH_ERRORS
 }
 
 bool integer(PyObject *o, int64_t &v) {

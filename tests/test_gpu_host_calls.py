@@ -154,3 +154,21 @@ def test_workspace_outlives_the_call(monkeypatch):
 	finally:
 		host.bind(*addresses)
 	assert freed == [0] and not table
+
+
+def test_an_exception_of_torch_reaches_the_caller(monkeypatch):
+	"""Out of memory inside a native call is raised there and then; the call is not made a second time in Python."""
+	layer = _layer(128, 8192, 128)
+	x = torch.randn(1 << 16, 128, device='cuda').half()
+	layer(x)          # (the workspace is there; the output took 1 GB)
+	torch.cuda.empty_cache()
+	again = []
+	monkeypatch.setattr(_lib, 'require_cuda', lambda *a: again.append(a))
+	total = torch.cuda.get_device_properties(0).total_memory
+	try:
+		torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (256 << 20)) / total)
+		with pytest.raises(torch.OutOfMemoryError):
+			layer(x)
+	finally:
+		torch.cuda.set_per_process_memory_fraction(1.0)
+	assert not again and layer(x).shape == (1 << 16, 8192)
