@@ -66,6 +66,7 @@ _SIGNATURES = {
 	'gptq_noalloc_scratch_bytes': (c_size_t, [c_int, c_int, c_int, c_int]),
 	'gptq_noalloc_status': (c_int, [c_int]),
 	'gptq_attn_prompt_scratch_bytes': (c_size_t, [c_int, c_int, c_int]),
+	'gptq_attn_prompt_full_scratch_bytes': (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
 	'gptq_attn_prompt_prepare': (c_int, [_P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, _P, c_int64, c_int64, _P, c_int64, c_int64, c_int, _P, _P, _P, c_size_t, _P]),
 	'gptq_attn_prompt': (c_int, [_P, c_int64, c_int64, c_int64, _P, _P, _P, c_int64, c_int64, c_int, c_int, c_int, c_int, c_int, ctypes.c_float, _P, _P, c_size_t, _P]),
 	'gptq_chain_supported': (c_int, [c_int, c_int, c_int, c_int, c_int]),
@@ -147,7 +148,7 @@ def host():
 			_host = _Ctypes
 			return _host
 		address = lambda name: ctypes.cast(getattr(l, name), c_void_p).value
-		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes',
+		module.bind(*map(address, ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_full_scratch_bytes',
 									 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')))
 		_host = module
 	return _host

@@ -32,7 +32,7 @@ decltype(&gptq_qmatmul) qmatmul_fn = nullptr;
 decltype(&gptq_gateup_silu) gateup_fn = nullptr;
 decltype(&gptq_qkv_rope) qkv_fn = nullptr;
 decltype(&gptq_dequantize) dequantize_fn = nullptr;
-decltype(&gptq_attn_prompt_scratch_bytes) attend_scratch = nullptr;
+decltype(&gptq_attn_prompt_full_scratch_bytes) attend_scratch = nullptr;
 decltype(&gptq_attn_prompt_prepare) attend_prepare = nullptr;
 decltype(&gptq_attn_prompt) attend_fn = nullptr;
 
@@ -293,7 +293,8 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 		if (pk && (!head_rows(*pk, b, H) || !head_rows(*pv, b, H) || pv->size(2) != past)) return nullptr;
 		// Long prompts whose mask rows start on 16 bytes are better off with the library kernel.  Whole block, this kernel / library, us: 32 heads, t = 1000 198 / 169,
 		// t = 400 of 5 sequences 312 / 295, t = 200 56 / 65, t = 64 40 / 65, t = 2 behind 100 36 / 80; 16 heads, t = 1200 98 / 105.  Rows off 16 bytes have to be
-		// copied for it: t = 701 behind 64 113 / 159, t = 1300 241 / 318, t = 2048 behind 1500 588 / 677.
+		// copied for it: t = 701 behind 64 110 / 143, t = 1300 behind 3 223 / 325, t = 2048 behind 1501 551 / 678; masks of the lowest value 117, 236, 577; biases that
+		// hide nothing 135, 286, 702.
 		const bool off = t > 128 && (mask->stride(2) % 8 != 0 || reinterpret_cast<uintptr_t>(mask->data_ptr()) % 16 != 0);
 		if (!off && b * H * t * S > (8 << 20)) return nullptr;
 		if (!c.workspace(a[0], w.K, w.N) || !c.gather(w, perm)) return nullptr;
@@ -301,7 +302,7 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 		const auto options = at::TensorOptions().dtype(at::kHalf).device(c.x->device());
 		const int shared = b == 1 || mask->stride(0) == 0, mask_b = shared ? 1 : (int)b;
 		const bool tiles = past > 0 || S > 128;          // (a launch less where there is next to nothing to skip)
-		const size_t need = tiles ? attend_scratch(mask_b, (int)t, (int)S) : 0;
+		const size_t need = tiles ? attend_scratch(mask_b, (int)b, (int)H, (int)t, (int)S) : 0;
 		at::Tensor q = at::empty({b, t, H, 128}, options), k = at::empty({b, H, S, 128}, options), v = at::empty({b, H, S, 128}, options), out = at::empty({b, t, H * 128}, options);
 		at::Tensor flags = at::empty({(int64_t)need}, options.dtype(at::kByte));
 		if ((q.key_set() | k.key_set() | v.key_set() | out.key_set() | flags.key_set() | pos.key_set()).has(c10::DispatchKey::Python)) return nullptr;
@@ -331,7 +332,7 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 	});
 }
 
-// bind(addresses of gptq_workspace_bytes, gptq_qmatmul, gptq_gateup_silu, gptq_qkv_rope, gptq_attn_prompt_scratch_bytes, _prepare, gptq_attn_prompt,
+// bind(addresses of gptq_workspace_bytes, gptq_qmatmul, gptq_gateup_silu, gptq_qkv_rope, gptq_attn_prompt_full_scratch_bytes, _prepare, gptq_attn_prompt,
 // gptq_dequantize)
 PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
 	if (n != 8) {

@@ -237,8 +237,12 @@ int gptq_embed_rmsnorm(const void *table, int64_t ldt, int64_t n_rows, const int
  *                              and head, rows of 128) to the front of k, v [b, heads, S, 128]
  *   gptq_attn_prompt           out [b, t, heads * 128] = softmax(q k^T scale + mask) v, scale > 0; a query that sees nothing gets zeros.  scratch NULL:
  *                              no tile of the mask has been classified
+ * Both take the same scratch with the same scratch_bytes.  With gptq_attn_prompt_full_scratch_bytes() of it (16-byte aligned) tiles that hold other values than
+ * 0 and -infinity are kept there in the order of their use, and tiles of large negative numbers only (at or below -8192) are left out where no key
+ * in them can have a weight; the smaller size holds the classes.  Results differ in nothing but the order in which tiles are added.
  */
 size_t gptq_attn_prompt_scratch_bytes(int b, int t, int S);
+size_t gptq_attn_prompt_full_scratch_bytes(int mask_b, int b, int heads, int t, int S);
 int gptq_attn_prompt_prepare(const void *mask, int64_t mask_sb, int64_t mask_st, int mask_b, int b, int heads, int t, int S,
                              const void *past_k, int64_t pk_sb, int64_t pk_sh, const void *past_v, int64_t pv_sb, int64_t pv_sh,
                              int past, void *k, void *v, void *scratch, size_t scratch_bytes, gptq_stream_t stream);

@@ -129,3 +129,82 @@ def test_calls_of_the_block(monkeypatch, b, t, past, kind, served):
 	assert attn(x, attention_mask=mask, past_key_value=kv)[2] is None
 	with pytest.raises(ValueError):
 		attn(x, attention_mask=torch.zeros((b, 1, t, past + t + 1), device='cuda').half(), past_key_value=kv)
+
+
+def _attend(q, k, v, mask, scale, full):
+	"""Output of the kernels [b, H, t, D] for q [b, t, H, D], whole k and v [b, H, S, D], and the classes of the tiles."""
+	(b, t, H, D), S = q.shape, k.shape[2]
+	mask_b = 1 if mask.stride(0) == 0 else b
+	l, P, st = _lib.lib(), _lib.ptr, _lib.stream_ptr(q.device)
+	classes = l.gptq_attn_prompt_scratch_bytes(mask_b, t, S)
+	need = l.gptq_attn_prompt_full_scratch_bytes(mask_b, b, H, t, S) if full else classes
+	scratch = torch.full((need + 64,), 0x5A, dtype=torch.uint8, device='cuda')
+	where = (P(mask), mask.stride(0), mask.stride(2), mask_b, b, H, t, S)
+	assert l.gptq_attn_prompt_prepare(*where, None, 0, 0, None, 0, 0, 0, P(k), P(v), P(scratch), need, st) == 0
+	out = torch.full((b, t, H * D), float('nan'), dtype=torch.float16, device='cuda')
+	assert l.gptq_attn_prompt(P(q), t * H * D, H * D, D, P(k), P(v), *where[:4], b, H, t, S, scale, P(out), P(scratch), need, st) == 0
+	assert bool((scratch[need:] == 0x5A).all())
+	return out.view(b, t, H, D).transpose(1, 2), scratch[:classes]
+
+
+@pytest.mark.parametrize('b,H,t,past', [(1, 2, 70, 0), (2, 3, 130, 70), (1, 2, 300, 129), (3, 1, 64, 577), (1, 1, 9, 8700)])
+@pytest.mark.parametrize('kind', ['lowest', 'both', 'ten thousand', 'blind rows', 'bias', 'strong'])
+def test_masks_of_finite_values(kind, b, H, t, past):
+	"""Masks as `transformers` builds them (the lowest fp16 value, its sum with itself, -10000), biases that hide nothing, and scores so large that
+	keys behind -9000 do count: with the full scratch, with the classes only, and against 64 bits."""
+	gen = torch.Generator(device='cuda').manual_seed(t + past)
+	S, D, low = t + past, 128, torch.finfo(torch.float16).min
+	rnd = lambda *shape: torch.randn(shape, generator=gen, device='cuda').half()
+	q, k, v = rnd(b, t, H, D), rnd(b, H, S, D), rnd(b, H, S, D)
+	hidden = torch.triu(torch.ones((t, S), dtype=torch.bool, device='cuda'), diagonal=past + 1)
+	mask = torch.zeros((b, 1, t, S), device='cuda', dtype=torch.float16).masked_fill(hidden, {'ten thousand': -1e4, 'strong': -9e3}.get(kind, low))
+	if kind in ('both', 'blind rows'):
+		for i in range(b):
+			mask[i, :, :, :(i + 1) * 37 % S] += low          # -inf where both
+	if kind == 'blind rows':
+		mask[:, :, t // 2:t // 2 + 3] = low
+	if kind == 'bias':
+		mask = rnd(b, 1, t, S) * 3
+	if kind == 'strong':          # whole heads' scores of up to +-20000, the visible ones at most zero
+		q[..., :], k[..., :] = 0, 0
+		q[..., 0] = 60.0
+		k[:, :, :past + t // 2, 0] = -0.25 * torch.rand((b, H, past + t // 2), generator=gen, device='cuda').half()
+		k[:, :, past + t // 2:, 0] = 4000.0 * torch.rand((b, H, t - t // 2), generator=gen, device='cuda').half()
+	scale = 0.09
+	s = q.transpose(1, 2).double() @ k.double().transpose(2, 3) * torch.tensor(scale, dtype=torch.float32).double().item() + mask.double()
+	blind = (s.amax(-1) < -3e4)
+	ref = torch.softmax(s, -1).nan_to_num(0.0) @ v.double()
+	# fp16 weights and result, and logits that are rounded in fp32: by 2^-9 at 65504, by 2^-11 at 20000, which is twice as much of a weight
+	bound = (1.1 * 2.0 ** -10 + torch.where(blind, 2.0 ** -8, 2.0 ** -10 if kind == 'strong' else 0.0)) * float(v.abs().max())
+	outs = [_attend(q, k, v, mask, scale, full) for full in (True, False)]
+	for out, _ in outs:
+		assert bool(((out.double() - ref).abs() <= bound[..., None]).all())
+	if kind in ('lowest', 'ten thousand', 'strong') and t > 128:
+		assert int((outs[0][1] == 3).sum()) > 0 and int((outs[1][1] == 3).sum()) == 0          # tiles that only the full scratch knows to be low
+
+
+def test_low_tiles_with_values_that_are_not_finite():
+	"""A query or key of infinities or NaN keeps the low tiles in: what a query sees of it does not depend on the scratch."""
+	b, H, t, D, low = 1, 2, 200, 128, torch.finfo(torch.float16).min
+	gen = torch.Generator(device='cuda').manual_seed(1)
+	q, k, v = (torch.randn(shape, generator=gen, device='cuda').half() for shape in ((b, t, H, D), (b, H, t, D), (b, H, t, D)))
+	mask = torch.zeros((b, 1, t, t), device='cuda', dtype=torch.float16).masked_fill(torch.triu(torch.ones((t, t), dtype=torch.bool, device='cuda'), diagonal=1), low)
+	q[0, 5, 0], k[0, 1, 190, 3] = float('nan'), INF
+	full, part = (_attend(q, k, v, mask, D ** -0.5, f)[0] for f in (True, False))
+	assert torch.equal(full.isnan(), part.isnan()) and bool(full[0, 0, 5].isnan().all()) and bool(full[0, 1, :190].isnan().any())
+	assert torch.allclose(full.nan_to_num(0), part.nan_to_num(0), atol=2e-3)
+
+
+def test_low_tiles_change_no_bit():
+	"""Left out or computed: the same bits (with a key whose norm keeps the tiles in, and which no query sees)."""
+	b, H, t, D, low = 1, 2, 333, 128, torch.finfo(torch.float16).min
+	gen = torch.Generator(device='cuda').manual_seed(2)
+	q, k, v = (torch.randn(shape, generator=gen, device='cuda').half() for shape in ((b, t, H, D), (b, H, t, D), (b, H, t, D)))
+	mask = torch.zeros((b, 1, t, t), device='cuda', dtype=torch.float16).masked_fill(torch.triu(torch.ones((t, t), dtype=torch.bool, device='cuda'), diagonal=1), low)
+	left_out = _attend(q, k, v, mask, D ** -0.5, True)[0]
+	k[:, :, t - 1] = 0
+	k[:, :, t - 1, 0] = 6e4
+	q[:, :t - 1, :, 0] = 0          # its score is zero for all queries in front, but the bound does not know
+	without = _attend(q, k.index_copy(2, torch.tensor([t - 1], device='cuda'), torch.zeros_like(k[:, :, :1])), v, mask, D ** -0.5, True)[0]
+	computed = _attend(q, k, v, mask, D ** -0.5, True)[0]
+	assert torch.equal(computed[:, :, :t - 1], without[:, :, :t - 1]) and bool(torch.isfinite(left_out).all())

@@ -135,7 +135,7 @@ def test_workspace_outlives_the_call(monkeypatch):
 	x = torch.randn(2, 256, device='cuda').half()
 	layer(x)
 	l, host = _lib.lib(), _lib.host()
-	names = ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_scratch_bytes', 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')
+	names = ('gptq_workspace_bytes', 'gptq_qmatmul', 'gptq_gateup_silu', 'gptq_qkv_rope', 'gptq_attn_prompt_full_scratch_bytes', 'gptq_attn_prompt_prepare', 'gptq_attn_prompt', 'gptq_dequantize')
 	addresses = [ctypes.cast(getattr(l, n), ctypes.c_void_p).value for n in names]
 	table = {(0, torch.cuda.current_stream().cuda_stream): torch.zeros(64 << 20, dtype=torch.uint8, device='cuda')}
 	freed = []
