@@ -12,10 +12,12 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/core/grad_mode.h>
 #include <ATen/ops/add.h>
+#include <ATen/ops/cat.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/index_select.h>
 #include <ATen/ops/matmul.h>
 #include <ATen/ops/mul.h>
+#include <ATen/ops/scaled_dot_product_attention.h>
 #include <ATen/ops/silu.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -295,20 +297,26 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 		// t = 400 of 5 sequences 312 / 295, t = 200 56 / 65, t = 64 40 / 65, t = 2 behind 100 36 / 80; 16 heads, t = 1200 98 / 105.  Rows off 16 bytes have to be
 		// copied for it: t = 701 behind 64 110 / 143, t = 1300 behind 3 223 / 325, t = 2048 behind 1501 551 / 678; masks of the lowest value 117, 236, 577; biases that
 		// hide nothing 135, 286, 702.
+		// One token over many keys, or a few tokens of many heads: a CTA per head and 64 queries has little to do per key, the library kernel splits the keys. GPU time, us:
+		// one token, 32 heads, 257 keys 32 / 33, 513 43 / 32, 1002 59 / 38, 4002 173 / 63, 16 sequences of 81 keys 45 / 55, of 256 82 / 65; 3 tokens, 4 sequences of 64 heads,
+		// 258 keys 84 / 87, 1004 145 / 139, 4004 410 / 380; 2 tokens, 4 sequences of 32 heads, 1003 keys 83 / 88.
+		const bool library = t == 1 ? S > 256 || b * H * S > 40000 : t <= 128 && b * H > 160 && S > 192;
 		const bool off = t > 128 && (mask->stride(2) % 8 != 0 || reinterpret_cast<uintptr_t>(mask->data_ptr()) % 16 != 0);
-		if (!off && b * H * t * S > (8 << 20)) return nullptr;
+		if (!off && !library && b * H * t * S > (8 << 20)) return nullptr;
 		if (!c.workspace(a[0], w.K, w.N) || !c.gather(w, perm)) return nullptr;
 		const at::Tensor pos = ids->reshape({-1}).to(at::kInt).contiguous();
 		const auto options = at::TensorOptions().dtype(at::kHalf).device(c.x->device());
 		const int shared = b == 1 || mask->stride(0) == 0, mask_b = shared ? 1 : (int)b;
-		const bool tiles = past > 0 || S > 128;          // (a launch less where there is next to nothing to skip)
+		const bool tiles = !library && (past > 0 || S > 128);          // (a launch less where there is next to nothing to skip)
 		const size_t need = tiles ? attend_scratch(mask_b, (int)b, (int)H, (int)t, (int)S) : 0;
-		at::Tensor q = at::empty({b, t, H, 128}, options), k = at::empty({b, H, S, 128}, options), v = at::empty({b, H, S, 128}, options), out = at::empty({b, t, H * 128}, options);
+		const int64_t rows = library ? t : S;          // (the library route concatenates: rows written between the cached ones are copied at half the speed)
+		at::Tensor q = at::empty({b, t, H, 128}, options), k = at::empty({b, H, rows, 128}, options), v = at::empty({b, H, rows, 128}, options), out;
+		if (!library) out = at::empty({b, t, H * 128}, options);
 		at::Tensor flags = at::empty({(int64_t)need}, options.dtype(at::kByte));
-		if ((q.key_set() | k.key_set() | v.key_set() | out.key_set() | flags.key_set() | pos.key_set()).has(c10::DispatchKey::Python)) return nullptr;
+		if ((q.key_set() | k.key_set() | v.key_set() | flags.key_set() | pos.key_set()).has(c10::DispatchKey::Python)) return nullptr;
 		int rc;
-		void *qp = q.data_ptr(), *kp = k.data_ptr(), *vp = v.data_ptr(), *op = out.data_ptr(), *fp = tiles ? flags.data_ptr() : nullptr;
-		const size_t skip = (size_t)past * 128 * 2;
+		void *qp = q.data_ptr(), *kp = k.data_ptr(), *vp = v.data_ptr(), *op = library ? nullptr : out.data_ptr(), *fp = tiles ? flags.data_ptr() : nullptr;
+		const size_t skip = library ? 0 : (size_t)past * 128 * 2;
 		const auto st = reinterpret_cast<gptq_stream_t>(c.stream);
 		Py_BEGIN_ALLOW_THREADS
 		rc = GPTQ_OK;
@@ -317,12 +325,16 @@ PyObject *attend(PyObject *, PyObject *const *a, Py_ssize_t n) {
 								pv ? pv->stride(0) : 0, pv ? pv->stride(1) : 0, (int)past, kp, vp, fp, need, st);
 		if (rc == GPTQ_OK)
 			rc = qkv_fn(c.rows_ptr(), words(w.qweight), words(w.qzeros), ptr(w.scales), nullptr, words(perm), ptr(cos), ptr(sin), words(&pos), (int)cos->size(0), qp, H * 128,
-						static_cast<char *>(kp) + skip, static_cast<char *>(vp) + skip, (int)t, H * S * 128, 128, S * 128, 0, (int)c.M, (int)w.K, (int)H, 128, (int)gs, w.K, c.ws,
+						static_cast<char *>(kp) + skip, static_cast<char *>(vp) + skip, (int)t, H * rows * 128, 128, rows * 128, 0, (int)c.M, (int)w.K, (int)H, 128, (int)gs, w.K, c.ws,
 						c.ws_bytes, st);
-		if (rc == GPTQ_OK)
+		if (rc == GPTQ_OK && !library)
 			rc = attend_fn(qp, t * H * 128, H * 128, 128, kp, vp, ptr(mask), mask->stride(0), mask->stride(2), mask_b, (int)b, (int)H, (int)t, (int)S, 0.08838834764831845f, op, fp, need, st);
 		Py_END_ALLOW_THREADS
 		if (rc != GPTQ_OK) return nullptr;
+		if (library) {
+			if (past) k = at::cat({*pk, k}, 2), v = at::cat({*pv, v}, 2);
+			out = at::scaled_dot_product_attention(q.transpose(1, 2), k, v, *mask).transpose(1, 2).reshape({b, t, H * 128});
+		}
 		PyObject *oo = THPVariable_Wrap(std::move(out)), *ko = THPVariable_Wrap(std::move(k)), *vo = THPVariable_Wrap(std::move(v));
 		PyObject *r = oo && ko && vo ? PyTuple_Pack(3, oo, ko, vo) : nullptr;
 		Py_XDECREF(oo);

@@ -208,3 +208,56 @@ def test_low_tiles_change_no_bit():
 	without = _attend(q, k.index_copy(2, torch.tensor([t - 1], device='cuda'), torch.zeros_like(k[:, :, :1])), v, mask, D ** -0.5, True)[0]
 	computed = _attend(q, k, v, mask, D ** -0.5, True)[0]
 	assert torch.equal(computed[:, :, :t - 1], without[:, :, :t - 1]) and bool(torch.isfinite(left_out).all())
+
+
+def _layer(K, N, seed, gs=128, act=False):
+	d = synth.quant_tensors(K, N, gs, seed)
+	layer = G.QuantLinear(4, gs, K, N, False)
+	layer.qweight, layer.qzeros, layer.scales = d['qweight'], d['qzeros'], d['scales']
+	layer = layer.cuda()
+	if act:
+		layer.set_g_idx((torch.arange(K, dtype=torch.int32) // gs)[torch.randperm(K, generator=torch.Generator().manual_seed(seed))])
+	return layer
+
+
+def _block(H, K=256, gs=128, act=False):
+	attn = G.QuantLlamaAttention(G.LlamaConfig(hidden_size=H * 128, num_attention_heads=H, max_position_embeddings=4096), _layer(H * 128, 3 * H * 128, 1, gs, act), _layer(H * 128, H * 128, 2), None)
+	return attn.cuda()
+
+
+def _both(monkeypatch, call):
+	"""call() as it is and with the native attention declined; what the native attention returned."""
+	host, seen = _lib.host(), []
+
+	class Counts:
+		qmatmul, gateup, qkv = host.qmatmul, host.gateup, host.qkv
+		attend = staticmethod(lambda *a: seen.append(host.attend(*a)) or seen[-1])
+
+	class Declines(Counts):
+		attend = staticmethod(lambda *a: None)
+	outs = []
+	for module in (Declines, Counts, Declines):          # (the first for the workspace)
+		with monkeypatch.context() as m:
+			m.setattr(_lib, '_host', module)
+			outs.append(call())
+	return outs[1], outs[2], seen[0]
+
+
+@pytest.mark.parametrize('H,b,t,past,library', [(2, 1, 1, 255, False), (2, 1, 1, 256, True), (2, 3, 1, 2000, True), (2, 79, 1, 252, False), (2, 80, 1, 252, True), (2, 80, 3, 220, False),
+												(2, 81, 3, 190, True), (2, 81, 3, 189, False), (2, 81, 128, 65, True), (2, 81, 129, 64, False)])
+@pytest.mark.parametrize('kind', ['shared', 'padded'])
+def test_one_token_and_many_heads(monkeypatch, kind, H, b, t, past, library):
+	"""Both sides of the lines beyond which the library's attention is the faster one: there the block gives its bits, as
+	without the native call."""
+	attn = _block(H)
+	gen = torch.Generator(device='cuda').manual_seed(past)
+	x = torch.randn((b, t, H * 128), generator=gen, device='cuda').half()
+	kv = tuple(torch.randn((b, H, past, 128), generator=gen, device='cuda').half() for _ in range(2))
+	mask = _mask(kind, b, t, t + past, gen)
+	new, old, seen = _both(monkeypatch, lambda: attn(x, attention_mask=mask, past_key_value=kv, use_cache=True))
+	assert seen is not None and all(torch.equal(a, c) and a.stride() == c.stride() for a, c in zip(new[2], old[2])) and new[0].shape == old[0].shape
+	same = torch.equal(new[0].nan_to_num(7.0), old[0].nan_to_num(7.0))
+	if library:
+		assert same
+	else:
+		assert float((new[0].float() - old[0].float()).abs().max()) <= 2e-3 * float(old[0].float().abs().max())
