@@ -261,3 +261,17 @@ def test_one_token_and_many_heads(monkeypatch, kind, H, b, t, past, library):
 		assert same
 	else:
 		assert float((new[0].float() - old[0].float()).abs().max()) <= 2e-3 * float(old[0].float().abs().max())
+
+
+@pytest.mark.parametrize('b,past,served', [(32, 902, True), (32, 904, False), (31, 904, True)])
+def test_portions_behind_a_long_cache(monkeypatch, b, past, served):
+	"""Mask rows off 16 bytes: 64 heads and more with eight times as many keys as queries are declined, as they were before there was a kernel."""
+	H, t = 2, 129
+	attn = _block(H)
+	gen = torch.Generator(device='cuda').manual_seed(past)
+	x = torch.randn((b, t, H * 128), generator=gen, device='cuda').half()
+	kv = tuple(torch.randn((b, H, past, 128), generator=gen, device='cuda').half() for _ in range(2))
+	mask = _mask('wide', b, t, t + past, gen)
+	new, old, seen = _both(monkeypatch, lambda: attn(x, attention_mask=mask, past_key_value=kv, use_cache=True))
+	assert (seen is not None) == served and all(torch.equal(a, c) for a, c in zip(new[2], old[2]))
+	assert float((new[0].float() - old[0].float()).abs().max()) <= (2e-3 * float(old[0].float().abs().max()) if served else 0.0)
