@@ -275,3 +275,57 @@ def test_portions_behind_a_long_cache(monkeypatch, b, past, served):
 	new, old, seen = _both(monkeypatch, lambda: attn(x, attention_mask=mask, past_key_value=kv, use_cache=True))
 	assert (seen is not None) == served and all(torch.equal(a, c) for a, c in zip(new[2], old[2]))
 	assert float((new[0].float() - old[0].float()).abs().max()) <= (2e-3 * float(old[0].float().abs().max()) if served else 0.0)
+
+
+@pytest.mark.parametrize('t,past,act,gs,ids', [(1, 2000, False, 128, None), (9, 31, True, 128, None), (40, 31, True, 128, torch.int64), (33, 96, False, 128, torch.int32), (16, 0, True, 64, torch.int64)])
+def test_native_attention_of_other_layers_and_positions(monkeypatch, t, past, act, gs, ids):
+	"""Act-order projections (gathered in the workspace up to 16 rows, ahead of the call above), given positions that are not a range, one query
+	behind 2000 keys: keys, values and outputs of the Python form; on a side stream and in a captured graph the same bits."""
+	b, H = 2, 2
+	attn = _block(H, gs=gs, act=act)
+	gen = torch.Generator(device='cuda').manual_seed(t)
+	x = torch.randn((b, t, H * 128), generator=gen, device='cuda').half()
+	kv = tuple(torch.randn((b, H, past, 128), generator=gen, device='cuda').half() for _ in range(2)) if past else None
+	mask = _mask('padded', b, t, t + past, gen)
+	pos = None if ids is None else torch.randint(0, 3000, (b, t), generator=gen, device='cuda').to(ids)
+	call = lambda: attn(x, attention_mask=mask, position_ids=pos, past_key_value=kv, use_cache=True)
+	new, old, seen = _both(monkeypatch, call)
+	assert seen is not None and all(torch.equal(a, c) for a, c in zip(new[2], old[2]))
+	assert float((new[0].nan_to_num(7.0).float() - old[0].nan_to_num(7.0).float()).abs().max()) <= 2e-3 * float(old[0].nan_to_num(0.0).float().abs().max())
+	side = torch.cuda.Stream()
+	side.wait_stream(torch.cuda.current_stream())
+	with torch.cuda.stream(side):
+		call()          # (workspace of this stream)
+		again = call()
+		graph = torch.cuda.CUDAGraph()
+		with torch.cuda.graph(graph, stream=side):
+			captured = call()
+		for y in (captured[0], *captured[2]):
+			y.zero_()
+		graph.replay()
+	side.synchronize()
+	for got in (again, captured):
+		assert torch.equal(got[0].nan_to_num(7.0), new[0].nan_to_num(7.0)) and all(torch.equal(a, c) for a, c in zip(got[2], new[2]))
+
+
+@pytest.mark.parametrize('case', ['groups of 32', 'no workspace', 'no tensor cores'])
+def test_native_attention_declines(monkeypatch, case):
+	"""... what it has no kernel or no workspace for; the block gives the results of the Python form."""
+	from gptq_triton_b200 import quant_linear
+	attn = _block(2, gs=32 if case == 'groups of 32' else 128)
+	x = torch.randn((1, 40, 256), device='cuda').half()
+	mask = _mask('padded', 1, 40, 40, None)
+	if case == 'no workspace':
+		monkeypatch.setattr(_lib, '_workspaces', {})
+	if case == 'no tensor cores':
+		monkeypatch.setattr(quant_linear, 'USE_TENSOR_CORE_KERNEL', False)
+	seen, host = [], _lib.host()
+
+	class Counts:
+		qmatmul, gateup, qkv = host.qmatmul, host.gateup, host.qkv
+		attend = staticmethod(lambda *a: seen.append(host.attend(*a)))
+	monkeypatch.setattr(_lib, '_host', Counts)
+	got = attn(x, attention_mask=mask, use_cache=True)
+	ref = attn(x, attention_mask=mask, use_cache=True, output_attentions=True)
+	assert seen == [None] and all(torch.equal(a, c) for a, c in zip(got[2], ref[2]))
+	assert float((got[0].nan_to_num(0).float() - ref[0].nan_to_num(0).float()).abs().max()) <= 4e-3 * float(ref[0].nan_to_num(0).float().abs().max())

@@ -172,3 +172,15 @@ def test_an_exception_of_torch_reaches_the_caller(monkeypatch):
 	finally:
 		torch.cuda.set_per_process_memory_fraction(1.0)
 	assert not again and layer(x).shape == (1 << 16, 8192)
+
+
+@pytest.mark.parametrize('M', [1, 16, 33])
+def test_qkv_of_an_act_order_layer(monkeypatch, M):
+	"""The QKV call with a permutation: gathered in the workspace up to 16 rows, in a tensor of its own above."""
+	H = 256
+	attn = G.QuantLlamaAttention(G.LlamaConfig(hidden_size=H, num_attention_heads=2), _layer(H, 3 * H, 128, act=True, seed=4), _layer(H, H, 128, seed=5), None)
+	x = torch.randn(1, M, H, device='cuda').half()
+	attn(x)
+	new, old, served = _both(monkeypatch, lambda: attn(x, use_cache=True))
+	assert len(served) == 2 and not any(s is None for s in served)
+	assert torch.equal(new[0], old[0]) and all(torch.equal(a, b) and a.stride() == b.stride() for a, b in zip(new[2], old[2]))
