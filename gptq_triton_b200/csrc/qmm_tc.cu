@@ -168,10 +168,12 @@ constexpr int TC_MAX_SPLITS = 8;       // portable cluster size
 // dequantisation (0.16 us at 32 rows in stages of two, 0.22 in stages of one) or the MMAs (0.38 us at 256 rows), a tile 2.5 us to start and
 // drain; with split K the partial tiles of the cluster are summed through distributed shared memory (4 us at 32 rows, 7 us at 256).  Against 4.8 us at 32
 // rows, a first fit on K >= 4096 only, us (dependent launches): 1024 -> 1024, 40 rows 5.9 -> 5.4; 2048 -> 6144, 17 rows 9.2 -> 8.4; 2048 -> 3072, 203 rows 10.1 -> 9.5;
-// 3072 -> 3072, 203 rows 11.4 -> 10.6; 2560 -> 7680, 100 rows 11.6 -> 10.7; 5504 -> 2048, 512 rows 16.6 -> 15.2; the wide layers choose as before.
-static double tc_cta_us(int nr, int splits, int kblocks) {
+// 3072 -> 3072, 203 rows 11.4 -> 10.6; 2560 -> 7680, 100 rows 11.6 -> 10.7; 5504 -> 2048, 512 rows 16.6 -> 15.2; the wide layers choose as before.  That holds for
+// one wave of clusters; of more the first fit is the better one (whole clusters have to leave before the next start): 8192 -> 10240, 64 rows 25.2 without a split, 26.8
+// with one, 8192 -> 2 x 5504, 100 rows 28.1 / 30.2.
+static double tc_cta_us(int nr, int splits, int kblocks, bool one_wave) {
 	const double t_kb = nr <= TC_PAIR_NR ? 0.14 + 0.00065 * nr : std::max(0.22 + 0.0002 * nr, 0.0015 * nr);
-	return kblocks * t_kb + (splits > 1 ? 3.5 + 0.014 * nr : 2.5);
+	return kblocks * t_kb + (splits == 1 ? 2.5 : one_wave ? 3.5 + 0.014 * nr : 4.5 + 0.01 * nr);
 }
 
 template <int EPI, int KP>
@@ -274,7 +276,8 @@ static int tc_launch_inst(TcParams p, cudaStream_t stream) {
 			const int n = slots_of(splits);
 			if (n <= 0) continue;
 			const long long ctas = (long long)mt * tiles * splits;
-			const double t = (double)((ctas + n - 1) / n) * tc_cta_us(nr, splits, per);
+			// (two tiles of 16 rows unpack the same weights twice for next to no MMAs: not for a tie; 2560 -> 2048, 17 rows 5.9 / 6.4)
+			const double t = (double)((ctas + n - 1) / n) * tc_cta_us(nr, splits, per, ctas <= n) * (mt > 1 && nr <= 16 ? 1.02 : 1.0);
 			if (t < best) {
 				best = t;
 				best_splits = splits;
