@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) attn_prepare_kernel(const PrepareParams p
 		const bool hidden = seen & 1u, open = seen & 2u, low = (seen & 4u) && p.tiles;
 		if (threadIdx.x == 0) p.flags[id] = hidden ? AP_HIDDEN : open ? AP_OPEN : low ? AP_LOW : AP_MIXED;
 		if (!p.tiles) return;
-		for (int i = id * 256 + threadIdx.x; i < p.n_norms; i += p.mask_ctas * 256) p.norms[i] = 0u;
+		for (long long i = id * 256ll + threadIdx.x; i < p.n_norms; i += p.mask_ctas * 256ll) p.norms[i] = 0u;
 		if (hidden || open) return;
 		// row r is entry h = r / 8 % 2 of the lanes 4 (r % 8) + 0 .. 3 of warp r / 16; a lane has columns 8 n + 2 tig, + 1 for n = 0 .. 7: four 16-byte units per h pair
 		const int r = threadIdx.x >> 2, quarter = threadIdx.x & 3, unit = (r >> 3 & 1) * 2 + (quarter >> 1);
